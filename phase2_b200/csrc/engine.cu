@@ -799,6 +799,21 @@ fail:
 	return NULL;
 }
 
+void p2_graph_drop(struct p2_dev *d, struct p2_graph *g)
+{
+	if (g->exec)
+		cudaGraphExecDestroy(g->exec);
+	if (g->d_cap) {
+		p2_scratch_free(g->d_recs, d->stream);
+	} else if (g->d_recs) {
+		cudaStreamSynchronize(d->stream);
+		cudaFree(g->d_recs);
+	}
+	free(g->passes);
+	free(g->recs);
+	memset(g, 0, sizeof *g);
+}
+
 extern "C" void p2d_destroy(struct p2_dev *d)
 {
 	if (!d)
@@ -821,14 +836,8 @@ extern "C" void p2d_destroy(struct p2_dev *d)
 	cudaFree(d->d_cm);
 	cudaFree(d->d_status);
 	cudaFreeHost(d->h_status);
-	for (int k = 0; k < P2_GRAPH_SLOTS; k++) {
-		struct p2_graph *g = &d->graphs[k];
-		if (g->exec)
-			cudaGraphExecDestroy(g->exec);
-		cudaFree(g->d_recs);
-		free(g->passes);
-		free(g->recs);
-	}
+	for (int k = 0; k < P2_GRAPH_SLOTS; k++)
+		p2_graph_drop(d, &d->graphs[k]);
 	if (d->t0)
 		cudaEventDestroy(d->t0);
 	if (d->t1)
@@ -1180,24 +1189,15 @@ static int launch_pass(struct p2_dev *d, const struct phase2_pass &p,
 	}
 }
 
-static int recs_reserve(struct p2_dev *d, size_t n)
+struct phase2_rot_rec *p2_stage_reserve(struct p2_dev *d, size_t n)
 {
-	if (n > d->d_recs_cap) {
-		size_t cap = d->d_recs_cap ? d->d_recs_cap : 1024;
-		while (cap < n)
-			cap *= 2;
-		CUDA_OK(cudaStreamSynchronize(d->stream), "sync before growth");
-		cudaFree(d->d_recs);
-		d->d_recs = NULL;
-		d->d_recs_cap = 0;
-		CUDA_OK(cudaMalloc((void **)&d->d_recs,
-				cap * sizeof(struct phase2_rot_rec)),
-			"alloc rotation records");
-		d->d_recs_cap = cap;
-	}
 	const int k = d->ring;
 	if (d->h_ev_live[k]) {
-		CUDA_OK(cudaEventSynchronize(d->h_ev[k]), "staging reuse");
+		if (cudaEventSynchronize(d->h_ev[k]) != cudaSuccess) {
+			log_error("staging reuse: %s",
+				cudaGetErrorString(cudaGetLastError()));
+			return NULL;
+		}
 		d->h_ev_live[k] = 0;
 	}
 	if (n > d->h_recs_cap[k]) {
@@ -1207,11 +1207,47 @@ static int recs_reserve(struct p2_dev *d, size_t n)
 		cudaFreeHost(d->h_recs[k]);
 		d->h_recs[k] = NULL;
 		d->h_recs_cap[k] = 0;
-		CUDA_OK(cudaMallocHost((void **)&d->h_recs[k],
-				cap * sizeof(struct phase2_rot_rec)),
-			"alloc pinned records");
+		if (cudaMallocHost((void **)&d->h_recs[k],
+			    cap * sizeof(struct phase2_rot_rec)) !=
+			cudaSuccess) {
+			d->h_recs[k] = NULL;
+			log_error("alloc pinned records: %s",
+				cudaGetErrorString(cudaGetLastError()));
+			return NULL;
+		}
 		d->h_recs_cap[k] = cap;
 	}
+	return d->h_recs[k];
+}
+
+int p2_stage_upload(struct p2_dev *d, void *dst, size_t bytes)
+{
+	const int k = d->ring;
+	CUDA_OK(cudaMemcpyAsync(dst, d->h_recs[k], bytes,
+			cudaMemcpyHostToDevice, d->stream),
+		"upload rotation records");
+	CUDA_OK(cudaEventRecord(d->h_ev[k], d->stream), "record staging");
+	d->h2d_bytes += bytes;
+	d->h_ev_live[k] = 1;
+	d->ring ^= 1;
+	return 0;
+}
+
+static int recs_reserve(struct p2_dev *d, size_t n)
+{
+	if (n <= d->d_recs_cap)
+		return 0;
+	size_t cap = d->d_recs_cap ? d->d_recs_cap : 1024;
+	while (cap < n)
+		cap *= 2;
+	CUDA_OK(cudaStreamSynchronize(d->stream), "sync before growth");
+	cudaFree(d->d_recs);
+	d->d_recs = NULL;
+	d->d_recs_cap = 0;
+	CUDA_OK(cudaMalloc((void **)&d->d_recs,
+			cap * sizeof(struct phase2_rot_rec)),
+		"alloc rotation records");
+	d->d_recs_cap = cap;
 	return 0;
 }
 
@@ -1267,7 +1303,7 @@ static struct p2_graph *graph_for(struct p2_dev *d,
 	for (int k = 0; k < P2_GRAPH_SLOTS; k++) {
 		struct p2_graph *g = &d->graphs[k];
 		if (g->hash == h && g->npass == npass && g->nrec == nrec &&
-			g->passes &&
+			g->passes && g->nsub == 0 &&
 			!memcmp(g->passes, passes, npass * sizeof *passes) &&
 			!memcmp(g->recs, recs, nrec * sizeof *recs)) {
 			g->used = d->graph_clock;
@@ -1311,15 +1347,7 @@ static struct p2_graph *graph_for(struct p2_dev *d,
 			lru = g;
 	}
 	/* first sighting: remember the plan in the least recently used slot */
-	if (lru->exec)
-		cudaGraphExecDestroy(lru->exec);
-	if (lru->d_recs) {
-		cudaStreamSynchronize(d->stream);
-		cudaFree(lru->d_recs);
-	}
-	free(lru->passes);
-	free(lru->recs);
-	memset(lru, 0, sizeof *lru);
+	p2_graph_drop(d, lru);
 	lru->passes = (struct phase2_pass *)malloc(npass * sizeof *passes);
 	lru->recs = (struct phase2_rot_rec *)malloc(nrec * sizeof *recs);
 	if (!lru->passes || !lru->recs) {
@@ -1338,31 +1366,36 @@ static struct p2_graph *graph_for(struct p2_dev *d,
 }
 
 extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec)
+	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
+	uint64_t plan_id)
 {
 	if (npass == 0)
 		return 0;
-	struct p2_graph *g = graph_for(d, passes, npass, recs, nrec);
-	if (!g) {
+	const bool resident = p2_resident_ok(d, passes[0].form);
+	struct p2_graph *g = resident
+		? NULL
+		: graph_for(d, passes, npass, recs, nrec);
+	if (!resident && !g) {
 		if (recs_reserve(d, nrec) < 0)
 			return -1;
-		const int k = d->ring;
-		memcpy(d->h_recs[k], recs, nrec * sizeof *recs);
-		CUDA_OK(cudaMemcpyAsync(d->d_recs, d->h_recs[k],
-				nrec * sizeof *recs, cudaMemcpyHostToDevice,
-				d->stream),
-			"upload rotation records");
-		CUDA_OK(cudaEventRecord(d->h_ev[k], d->stream),
-			"record staging");
-		d->h2d_bytes += nrec * sizeof *recs;
-		d->h_ev_live[k] = 1;
-		d->ring ^= 1;
+		struct phase2_rot_rec *stage = p2_stage_reserve(d, nrec);
+		if (!stage)
+			return -1;
+		memcpy(stage, recs, nrec * sizeof *recs);
+		if (p2_stage_upload(d, d->d_recs, nrec * sizeof *recs) < 0)
+			return -1;
 	}
 
-	if (d->timing)
+	if (d->timing && !resident)
 		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	long launches;
-	if (g) {
+	if (resident) {
+		/* counted as one state round trip a pass, as planned */
+		if (p2_resident_run(d, passes, npass, recs, nrec, plan_id) < 0)
+			return -1;
+		d->launches++;
+		launches = (long)npass;
+	} else if (g) {
 		CUDA_OK(cudaGraphLaunch(g->exec, d->stream), "graph launch");
 		d->graph_replays++;
 		d->status_pending |= g->status;
@@ -1373,7 +1406,7 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	CUDA_OK(cudaGetLastError(), "pass launch");
 	d->passes += npass;
 	d->sweeps += (uint64_t)launches;
-	d->launches += (uint64_t)launches;
+	d->launches += resident ? 0 : (uint64_t)launches;
 	d->rotations += nrec;
 	if (d->timing) {
 		CUDA_OK(cudaEventRecord(d->t1, d->stream), "timing stop");

@@ -30,6 +30,11 @@ struct p2_graph {
 	struct phase2_rot_rec *d_recs; /* records read by the graph */
 	cudaGraphExec_t exec;
 	size_t nlaunch; /* kernel launches in the graph */
+	/* resident registers (resident.cu): d_recs holds the flush's repacked
+	 * records and its nsub sub-passes, d_cap bytes from the pool */
+	size_t d_cap;
+	uint32_t nsub;
+	uint64_t plan_id; /* the caller's number of this plan (0: none) */
 	int status;     /* the graph holds kernels that write d_status */
 	uint64_t used;
 };
@@ -140,6 +145,23 @@ void p2_batch_launch(int kind, unsigned grid, cudaStream_t stream,
 	const uint64_t *widx, const double *wval, const uint64_t *gidx,
 	double2 *gout, struct p2_bctl *ctl, unsigned int *status,
 	const double *cum);
+
+/* engine.cu: pinned staging for `n` records of 32 bytes (double buffered;
+ * NULL on failure), and the copy of its first `bytes` to device memory. */
+struct phase2_rot_rec *p2_stage_reserve(struct p2_dev *d, size_t n);
+int p2_stage_upload(struct p2_dev *d, void *dst, size_t bytes);
+
+/* engine.cu: release a plan slot (graph or resident plan) and clear it. */
+void p2_graph_drop(struct p2_dev *d, struct p2_graph *g);
+
+/* resident.cu: whether a register's flush of this form runs as one launch
+ * on the register held in shared memory, and that launch (between the
+ * timing events; the caller counts it).  plan_id: nonzero and the same for
+ * flushes with the same passes and records. */
+bool p2_resident_ok(const struct p2_dev *d, int form);
+int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
+	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
+	uint64_t plan_id);
 
 /* lift_bulk.cu: one FP32 pass of the FP64-arithmetic form on a kernel
  * whose next cosets are staged in shared memory, by bulk copies (variant

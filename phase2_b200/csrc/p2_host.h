@@ -61,6 +61,7 @@ struct p2_qreg {
 	size_t plan_qlen, plan_qcap;
 	long plan_np;
 	int plan_span, plan_rots, plan_form, plan_sweep;
+	uint64_t plan_id; /* number of the plan held in passes/recs */
 };
 
 /* Sticky error of a register (0 ok, -1 failed). */

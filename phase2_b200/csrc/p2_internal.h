@@ -66,9 +66,11 @@ int p2d_get(struct p2_dev *d, const uint64_t *idx, double *z, size_t n);
 int p2d_get_state(struct p2_dev *d, double *out);
 int p2d_set_state(struct p2_dev *d, const double *in);
 
-/* Upload `nrec` records and launch `npass` passes on the stream. */
+/* Upload `nrec` records and launch `npass` passes on the stream.  plan_id:
+ * a number of this plan, nonzero and never used for another plan of the
+ * register (a plan run again under its number is not compared). */
 int p2d_run(struct p2_dev *d, const struct phase2_pass *passes, size_t npass,
-	const struct phase2_rot_rec *recs, size_t nrec);
+	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id);
 
 int p2d_norm2(struct p2_dev *d, double *out);
 int p2d_inner_dense(struct p2_dev *d, const double *trial, double out[2]);

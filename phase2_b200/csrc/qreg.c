@@ -210,13 +210,14 @@ static int drain_rotations(struct qreg *reg)
 			b->max_rots, P2_DEFAULT_PAD_SPAN, form, swk, swl,
 			b->passes, b->recs);
 		remember_plan(b, np, form, sweep);
+		b->plan_id++;
 	}
 	if (np >= 0 && b->rec) {
 		if (p2_prog_plan(b->rec, b->passes, (size_t)np, b->recs,
 			    b->qlen, same) < 0)
 			b->error = -1;
 	} else if (np < 0 || p2d_run(b->dev, b->passes, (size_t)np, b->recs,
-				    b->qlen) < 0) {
+				    b->qlen, b->plan_id) < 0) {
 		log_error("qreg: %zu rotations failed", b->qlen);
 		b->error = -1;
 	}

@@ -1,0 +1,505 @@
+/*
+ * resident.cu -- small registers held on chip: one launch runs a whole
+ * flush.
+ *
+ * A register of up to 14 qubits is at most 256 KiB (as complex doubles): one
+ * block, or one thread-block cluster, holds it in shared memory, so the
+ * passes of a flush need no kernel boundary between them, only a barrier.
+ * The pass kernels spend 5 us on such a pass of 5 random strings: a launch,
+ * one or a few blocks of cold code (64 cases of 32 unrolled slots), and one
+ * warp a scheduler whose FP64 operations wait for one another.  Here a
+ * sub-pass of 3 strings takes 1 us, bound by latencies (ncu, 10 qubits: one
+ * instruction in 4 cycles and scheduler, 1.7 of them fixed-latency waits;
+ * 144 warp instructions a rotation, 48 of them FP64 products and sums).
+ * ns a rotation, 10 / 12 / 14 qubits: random strings 322 / 608 / 921
+ * (pass kernels 943 / 1122 / 1133), excitation groups of 8 strings 169 /
+ * 204 / 234 (402 / 430 / 430).
+ */
+#include <cuda_runtime.h>
+
+#include <stdint.h>
+#include <stdlib.h>
+#include <string.h>
+
+#define LOG_SUBSYS "engine"
+#include "log.h"
+
+/* all four pairs of a coset step by step: a warp is nearly alone on its
+ * scheduler here, so independent FP64 operations have to come from it */
+#define P2_ROT_GROUP 4
+#define P2_LIFT_GROUP 4
+#include "p2_kernels.cuh"
+#include "sub_core.h"
+
+#define P2_RES_MIN_QB 3
+#define P2_RES_MAX_QB 14
+#define P2_RES_TPB 256
+#define P2_RES_SLOTS (1 << P2_SUB_SPAN)
+#define P2_RES_SMEM (16 << 11) /* the most amplitudes of a block, 2^11 */
+
+/* ---- shared memory of the cluster --------------------------------------- */
+
+template <bool CL>
+__device__ __forceinline__ uint32_t p2_res_addr(uint32_t base, uint32_t pos,
+	uint32_t kc)
+{
+	uint32_t a = base + ((pos & ((1u << kc) - 1u)) << 4);
+	if constexpr (CL) {
+		const uint32_t rank = pos >> kc;
+		asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a)
+			: "r"(a), "r"(rank));
+	}
+	return a;
+}
+
+template <bool CL>
+__device__ __forceinline__ void p2_res_ld(uint32_t a, double &re, double &im)
+{
+	if constexpr (CL)
+		asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
+			: "=d"(re), "=d"(im) : "r"(a) : "memory");
+	else
+		asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
+			: "=d"(re), "=d"(im) : "r"(a) : "memory");
+}
+
+template <bool CL>
+__device__ __forceinline__ void p2_res_st(uint32_t a, double re, double im)
+{
+	if constexpr (CL)
+		asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};"
+			:: "r"(a), "d"(re), "d"(im) : "memory");
+	else
+		asm volatile("st.shared.v2.f64 [%0], {%1, %2};"
+			:: "r"(a), "d"(re), "d"(im) : "memory");
+}
+
+template <bool CL> __device__ __forceinline__ void p2_res_barrier()
+{
+	if constexpr (CL)
+		asm volatile("barrier.cluster.arrive.release.aligned;\n"
+			     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+	else
+		__syncthreads();
+}
+
+/* The rotation (key) on a coset of 8 slots: the exact FP64 update, or the
+ * lifted one in FP64. */
+template <bool X, int K>
+__device__ __forceinline__ void p2_sub_rot(double (&re)[P2_RES_SLOTS],
+	double (&im)[P2_RES_SLOTS], double c, double s, uint32_t sm)
+{
+	if constexpr (X)
+		p2_rot_lift<P2_SUB_SPAN, (K >> 1), (K & 1)>(re, im, c, s, sm);
+	else
+		p2_rot<P2_SUB_SPAN, (K >> 1), (K & 1)>(re, im, c, s, sm, 0u);
+}
+
+#define P2_CASE_S(K)                                                           \
+	case K:                                                                \
+		p2_sub_rot<X, K>(re, im, q.c, q.s, sm);                        \
+		break;
+
+template <bool X>
+__device__ __forceinline__ void p2_sub_apply(const struct p2_sub_rec &q,
+	double (&re)[P2_RES_SLOTS], double (&im)[P2_RES_SLOTS], uint32_t sm)
+{
+	switch (q.key) {
+		P2_CASE_S(0) P2_CASE_S(1) P2_CASE_S(2) P2_CASE_S(3)
+		P2_CASE_S(4) P2_CASE_S(5) P2_CASE_S(6) P2_CASE_S(7)
+		P2_CASE_S(8) P2_CASE_S(9) P2_CASE_S(10) P2_CASE_S(11)
+		P2_CASE_S(12) P2_CASE_S(13) P2_CASE_S(14) P2_CASE_S(15)
+	default:
+		break;
+	}
+}
+#undef P2_CASE_S
+
+/* ---- the kernel ---------------------------------------------------------- */
+
+/* Sub-passes whose records are on their way or in use, and headers held:
+ * a sub-pass can be shorter than the latency of a copy from L2. */
+#define P2_RES_STAGES 4
+#define P2_RES_HDRS 8
+
+/* Start the copy of sub-pass j's records (one commit group a call). */
+__device__ __forceinline__ void p2_res_stage(uint32_t j, uint32_t nsub,
+	const struct p2_sub *hdr,
+	struct p2_sub_rec (*srec)[P2_SUB_ROTS],
+	const struct p2_sub_rec *__restrict__ recs, uint32_t tid, uint32_t nt)
+{
+	if (j < nsub) {
+		const struct p2_sub &h = hdr[j % P2_RES_HDRS];
+		const uint32_t dst = (uint32_t)__cvta_generic_to_shared(
+			&srec[j % P2_RES_STAGES][0]);
+		const unsigned char *const src =
+			(const unsigned char *)(recs + h.rot_off);
+		for (uint32_t k = tid; k < 2u * h.nrot; k += nt)
+			p2_cp16(dst + 16 * k, src + 16 * k);
+	}
+	p2_cp_commit();
+}
+
+/*
+ * One cluster (CL) or block: blocks of 2^kc amplitudes each.  A sub-pass
+ * is one trip of every amplitude through registers (8 a thread) and one
+ * barrier; the records of the next sub-pass and the header after it are
+ * copied to shared memory meanwhile.  The state is held as complex doubles
+ * whatever its precision: FP32 states round at the end of each pass, where
+ * the pass kernels do.
+ */
+template <typename ST, bool X, bool CL>
+__global__ void __launch_bounds__(P2_RES_TPB) k_resident(ST *__restrict__ st,
+	uint32_t nqb, uint32_t kc, const struct p2_sub *__restrict__ subs,
+	uint32_t nsub, const struct p2_sub_rec *__restrict__ recs)
+{
+	extern __shared__ __align__(16) unsigned char p2_res_dyn[];
+	__shared__ __align__(16) struct p2_sub hdr[P2_RES_HDRS];
+	__shared__ __align__(16) struct p2_sub_rec srec[P2_RES_STAGES]
+						       [P2_SUB_ROTS];
+	const uint32_t tid = threadIdx.x, nt = blockDim.x;
+	const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(p2_res_dyn);
+	const uint32_t rank = CL ? blockIdx.x : 0u;
+	const uint32_t mine = 1u << kc, first = rank << kc;
+	const uint32_t t = rank * nt + tid;
+	const bool active = t < (1u << (nqb - P2_SUB_SPAN));
+
+	/* headers of the first sub-passes (the reads of the loop below), the
+	 * block's amplitudes, then the records of the first stages */
+	for (uint32_t k = tid; k < 4 * P2_RES_HDRS && k < 4 * nsub; k += nt)
+		p2_cp16((uint32_t)__cvta_generic_to_shared(hdr) + 16 * k,
+			(const unsigned char *)subs + 16 * k);
+	for (uint32_t i = tid; i < mine; i += nt) {
+		double re, im;
+		p2_ld(st, first + i, re, im);
+		p2_res_st<false>(p2_res_addr<false>(sbase,
+				 p2_sub_swz(first + i), kc), re, im);
+	}
+	p2_cp_commit();
+	p2_cp_wait<0>();
+	__syncthreads();
+	for (uint32_t j = 0; j < P2_RES_STAGES - 1; ++j)
+		p2_res_stage(j, nsub, hdr, srec, recs, tid, nt);
+	p2_cp_wait<P2_RES_STAGES - 2>();
+	p2_res_barrier<CL>();
+
+	for (uint32_t i = 0; i < nsub; ++i) {
+		const struct p2_sub &h = hdr[i % P2_RES_HDRS];
+		const struct p2_sub_rec *const q0 = srec[i % P2_RES_STAGES];
+		/* the header whose records are staged P2_RES_STAGES - 1 rounds
+		 * from now, into the place of the one just done */
+		if (i > 0 && i + P2_RES_HDRS - 1 < nsub && tid < 4)
+			p2_cp16((uint32_t)__cvta_generic_to_shared(
+					&hdr[(i - 1) % P2_RES_HDRS]) + 16 * tid,
+				(const unsigned char *)(subs + i +
+					P2_RES_HDRS - 1) + 16 * tid);
+		p2_res_stage(i + P2_RES_STAGES - 1, nsub, hdr, srec, recs, tid,
+			nt);
+		if (active) {
+			uint32_t x = t;
+#pragma unroll
+			for (int k = 0; k < P2_SUB_SPAN; ++k) {
+				const uint32_t p = h.piv[k];
+				x = ((x >> p) << (p + 1)) | (x & ((1u << p) - 1u));
+			}
+			if constexpr (X) {
+				const uint32_t x0 = x;
+#pragma unroll
+				for (int k = 0; k < P2_SUB_SPAN; ++k)
+					x ^= (0u - p2_parity(x0 & h.orient[k])) &
+						h.slot[k];
+			}
+			const uint32_t px = p2_sub_swz(x);
+			uint32_t addr[P2_RES_SLOTS];
+			double re[P2_RES_SLOTS], im[P2_RES_SLOTS];
+#pragma unroll
+			for (int u = 0; u < P2_RES_SLOTS; ++u) {
+				uint32_t p = px;
+#pragma unroll
+				for (int k = 0; k < P2_SUB_SPAN; ++k)
+					if (u >> k & 1)
+						p ^= h.pslot[k];
+				addr[u] = p2_res_addr<CL>(sbase, p, kc);
+				p2_res_ld<CL>(addr[u], re[u], im[u]);
+			}
+			const uint32_t nrot = h.nrot;
+			for (uint32_t r = 0; r < nrot; ++r) {
+				const struct p2_sub_rec q = q0[r];
+				p2_sub_apply<X>(q, re, im,
+					(uint32_t)q.sm ^ (0u - p2_parity(x & q.z)));
+			}
+			if (X && (h.flags & P2_SUB_LAST)) {
+				const uint32_t neg = h.flags & P2_SUB_NEG
+					? 0x80000000u : 0u;
+#pragma unroll
+				for (int u = 0; u < P2_RES_SLOTS; ++u) {
+					re[u] = (double)__double2float_rn(
+						p2_sgn(re[u], neg));
+					im[u] = (double)__double2float_rn(
+						p2_sgn(im[u], neg));
+				}
+			}
+#pragma unroll
+			for (int u = 0; u < P2_RES_SLOTS; ++u)
+				p2_res_st<CL>(addr[u], re[u], im[u]);
+		}
+		p2_cp_wait<P2_RES_STAGES - 2>();
+		p2_res_barrier<CL>();
+	}
+	p2_cp_wait<0>();
+	for (uint32_t i = tid; i < mine; i += nt) {
+		double re, im;
+		p2_res_ld<false>(p2_res_addr<false>(sbase,
+				 p2_sub_swz(first + i), kc), re, im);
+		p2_st(st, first + i, re, im);
+	}
+}
+
+/* ---- host side ----------------------------------------------------------- */
+
+/*
+ * log2 of the blocks of a register's cluster: one block up to 11 qubits,
+ * where a second block only adds the cluster barrier and remote shared
+ * memory (11 qubits, random strings, ns a rotation: 399 on one block, 592
+ * on two); 8 at 12 qubits (608; 645 on one, 731 on four), 16 at 13 and 14
+ * (651 and 921; the pass kernels 1112 and 1133).  At 15 qubits the traffic
+ * between the blocks bounds a sub-pass (1583) and the pass kernels are
+ * faster (1122).
+ */
+static uint32_t res_log_blocks(uint32_t nqb)
+{
+	return nqb <= 11 ? 0 : nqb == 12 ? 3 : 4;
+}
+
+/* 64-bit words, four chains (n a multiple of 8). */
+static uint64_t hash_words(uint64_t h, const void *p, size_t n)
+{
+	const unsigned char *b = (const unsigned char *)p;
+	uint64_t c[4] = { h, ~h, h << 7, h >> 9 };
+	size_t i = 0;
+	for (; i + 32 <= n; i += 32) {
+		uint64_t w[4];
+		memcpy(w, b + i, 32);
+		for (int k = 0; k < 4; k++) {
+			c[k] = (c[k] ^ w[k]) * UINT64_C(0x9e3779b97f4a7c15);
+			c[k] ^= c[k] >> 29;
+		}
+	}
+	for (; i + 8 <= n; i += 8) {
+		uint64_t w;
+		memcpy(&w, b + i, 8);
+		c[0] = (c[0] ^ w) * UINT64_C(0x9e3779b97f4a7c15);
+		c[0] ^= c[0] >> 29;
+	}
+	for (int k = 1; k < 4; k++)
+		c[0] = (c[0] ^ c[k]) * UINT64_C(0x9e3779b97f4a7c15) ^
+			(c[k] >> 31);
+	return c[0];
+}
+
+/*
+ * The device copy of a flush's sub-passes: found among the last
+ * P2_GRAPH_SLOTS plans of the register by plan id (the same flush again) or
+ * by content, or built and uploaded into the least recently used slot
+ * (stream order keeps the copy behind the launches that read the slot).
+ * *hit: found.  NULL on failure.
+ */
+static struct p2_graph *res_plan(struct p2_dev *d,
+	const struct phase2_pass *passes, size_t npass,
+	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id,
+	bool *hit)
+{
+	struct p2_graph *lru = &d->graphs[0];
+	d->graph_clock++;
+	*hit = true;
+	for (int k = 0; k < P2_GRAPH_SLOTS; k++) {
+		struct p2_graph *g = &d->graphs[k];
+		if (plan_id && g->nsub && g->plan_id == plan_id) {
+			g->used = d->graph_clock;
+			return g;
+		}
+	}
+	uint64_t h = hash_words(UINT64_C(0xcbf29ce484222325), passes,
+		npass * sizeof *passes);
+	h = hash_words(h, recs, nrec * sizeof *recs);
+	for (int k = 0; k < P2_GRAPH_SLOTS; k++) {
+		struct p2_graph *g = &d->graphs[k];
+		if (g->nsub && g->hash == h && g->npass == npass &&
+			g->nrec == nrec &&
+			!memcmp(g->passes, passes, npass * sizeof *passes) &&
+			!memcmp(g->recs, recs, nrec * sizeof *recs)) {
+			g->used = d->graph_clock;
+			g->plan_id = plan_id;
+			return g;
+		}
+		if (g->used < lru->used)
+			lru = g;
+	}
+	*hit = false;
+	if (lru->d_cap) {
+		/* keep the device buffer of a resident plan */
+		free(lru->passes);
+		free(lru->recs);
+		lru->nsub = 0;
+	} else {
+		p2_graph_drop(d, lru);
+	}
+	lru->passes = (struct phase2_pass *)malloc(npass * sizeof *passes);
+	lru->recs = (struct phase2_rot_rec *)malloc(nrec * sizeof *recs);
+	lru->hash = h;
+	lru->npass = npass;
+	lru->nrec = nrec;
+	lru->plan_id = 0;
+	lru->used = 0;
+	if (!lru->passes || !lru->recs)
+		goto fail;
+	memcpy(lru->passes, passes, npass * sizeof *passes);
+	memcpy(lru->recs, recs, nrec * sizeof *recs);
+	{
+		/* staging: sub-passes from the end of the records' area on (at
+		 * most one a rotation) */
+		struct phase2_rot_rec *stage =
+			p2_stage_reserve(d, 3 * nrec);
+		if (!stage)
+			goto fail;
+		struct p2_sub_rec *const sr = (struct p2_sub_rec *)stage;
+		struct p2_sub *const ss = (struct p2_sub *)(sr + nrec);
+		uint32_t n = 0;
+		for (size_t i = 0; i < npass; i++)
+			n += p2_sub_split(&passes[i], recs + passes[i].rot_off,
+				d->nqb, passes[i].rot_off, ss + n,
+				sr + passes[i].rot_off);
+		const size_t bytes = nrec * sizeof *sr + n * sizeof *ss;
+		if (bytes > lru->d_cap) {
+			p2_scratch_free(lru->d_recs, d->stream);
+			lru->d_recs = NULL;
+			lru->d_cap = 0;
+			if (p2_scratch_alloc((void **)&lru->d_recs, bytes,
+				    d->stream) != cudaSuccess) {
+				lru->d_recs = NULL;
+				goto fail;
+			}
+			lru->d_cap = bytes;
+		}
+		if (p2_stage_upload(d, lru->d_recs, bytes) < 0)
+			goto fail;
+		lru->nsub = n;
+	}
+	lru->plan_id = plan_id;
+	lru->used = d->graph_clock;
+	return lru;
+fail:
+	log_error("resident plan: out of memory");
+	cudaGetLastError();
+	p2_graph_drop(d, lru);
+	return NULL;
+}
+
+/* Largest cluster the kernel can be launched with on this device (blocks of
+ * 128 threads and 16 KiB), once per instantiation; 0 when it cannot be
+ * configured. */
+template <typename ST, bool X, bool CL> static unsigned res_clusters(void)
+{
+	static unsigned most; /* 1 + the answer */
+	unsigned m = __atomic_load_n(&most, __ATOMIC_ACQUIRE);
+	if (m)
+		return m - 1;
+	unsigned best = 0;
+	if (cudaFuncSetAttribute(k_resident<ST, X, CL>,
+		    cudaFuncAttributeMaxDynamicSharedMemorySize,
+		    P2_RES_SMEM) == cudaSuccess) {
+		best = 1;
+		if (CL && cudaFuncSetAttribute(k_resident<ST, X, CL>,
+				  cudaFuncAttributeNonPortableClusterSizeAllowed,
+				  1) != cudaSuccess)
+			best = 0;
+		for (unsigned c = 16; CL && best == 1 && c > 1; c /= 2) {
+			cudaLaunchConfig_t cfg;
+			cudaLaunchAttribute at[1];
+			memset(&cfg, 0, sizeof cfg);
+			at[0].id = cudaLaunchAttributeClusterDimension;
+			at[0].val.clusterDim.x = c;
+			at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+			cfg.gridDim = dim3(c);
+			cfg.blockDim = dim3(128);
+			cfg.dynamicSmemBytes = 16 << 10;
+			cfg.attrs = at;
+			cfg.numAttrs = 1;
+			int n = 0;
+			if (cudaOccupancyMaxActiveClusters(&n,
+				    k_resident<ST, X, CL>, &cfg) ==
+					cudaSuccess && n > 0)
+				best = c;
+		}
+	}
+	cudaGetLastError();
+	__atomic_store_n(&most, best + 1, __ATOMIC_RELEASE);
+	return best;
+}
+
+bool p2_resident_ok(const struct p2_dev *d, int form)
+{
+	if (d->nqb < P2_RES_MIN_QB || d->nqb > P2_RES_MAX_QB ||
+		form == PHASE2_FORM_LIFTED_F32)
+		return false;
+	const uint32_t lb = res_log_blocks(d->nqb);
+	const unsigned most = d->prec == PHASE2_PREC_FP64
+		? (lb ? res_clusters<double2, false, true>()
+		      : res_clusters<double2, false, false>())
+		: (lb ? res_clusters<float2, true, true>()
+		      : res_clusters<float2, true, false>());
+	return most >= (1u << lb);
+}
+
+template <typename ST, bool X, bool CL>
+static int res_launch(struct p2_dev *d, uint32_t lb, const struct p2_graph *g)
+{
+	const uint32_t kc = d->nqb - lb;
+	const size_t smem = (size_t)16 << kc;
+	uint32_t tpb = 1u << (d->nqb - P2_SUB_SPAN - lb);
+	if (tpb < 32)
+		tpb = 32;
+	cudaLaunchConfig_t cfg;
+	cudaLaunchAttribute at[1];
+	memset(&cfg, 0, sizeof cfg);
+	cfg.gridDim = dim3(1u << lb);
+	cfg.blockDim = dim3(tpb);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = d->stream;
+	if (CL) {
+		at[0].id = cudaLaunchAttributeClusterDimension;
+		at[0].val.clusterDim.x = 1u << lb;
+		at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+		cfg.attrs = at;
+		cfg.numAttrs = 1;
+	}
+	const struct p2_sub_rec *sr = (const struct p2_sub_rec *)g->d_recs;
+	CUDA_OK(cudaLaunchKernelEx(&cfg, k_resident<ST, X, CL>, (ST *)d->state,
+			d->nqb, kc, (const struct p2_sub *)(sr + g->nrec),
+			g->nsub, sr),
+		"resident launch");
+	return 0;
+}
+
+int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
+	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
+	uint64_t plan_id)
+{
+	bool hit;
+	struct p2_graph *g = res_plan(d, passes, npass, recs, nrec, plan_id,
+		&hit);
+	if (!g)
+		return -1;
+	d->graph_replays += hit;
+	const uint32_t lb = res_log_blocks(d->nqb);
+	if (d->timing)
+		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
+	int rc;
+	if (d->prec == PHASE2_PREC_FP64)
+		rc = lb ? res_launch<double2, false, true>(d, lb, g)
+			: res_launch<double2, false, false>(d, lb, g);
+	else
+		rc = lb ? res_launch<float2, true, true>(d, lb, g)
+			: res_launch<float2, true, false>(d, lb, g);
+	return rc;
+}
