@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include <float.h>
+#include <pthread.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -713,65 +714,85 @@ static int io_reserve(struct p2_dev *d, size_t n)
 	return 0;
 }
 
-extern "C" struct p2_dev *p2d_create(uint32_t nqb, int prec)
+/* ---- register shells ------------------------------------------------------ */
+
+/*
+ * A register's stream, events, status words, staging and small buffers.
+ * Creating and freeing them costs 3 ms where no other register keeps the
+ * allocator's blocks alive (a whole 10-qubit run computes for 0.1 ms), so
+ * a destroyed register leaves them for the next one: at most
+ * P2_SHELLS of them, each holding at most P2_SHELL_BYTES of buffers, per
+ * context, given back by p2d_release (world_free).
+ */
+#define P2_SHELLS 32
+#define P2_SHELL_BYTES ((size_t)2 << 20)
+
+static pthread_mutex_t shell_lock = PTHREAD_MUTEX_INITIALIZER;
+static struct p2_dev *shells[P2_SHELLS];
+static int nshells;
+
+/* A number that differs between a device's contexts (a device reset makes
+ * a new one, in which kept handles mean nothing); 0 where it is unknown. */
+static uint64_t context_id(void)
 {
-	if (nqb == 0 || nqb > 40) {
-		log_error("p2d_create: nqb=%u out of range", nqb);
-		return NULL;
+	typedef int (*get_id)(void *, unsigned long long *);
+	static get_id fn;
+	static int looked;
+	if (!__atomic_load_n(&looked, __ATOMIC_ACQUIRE)) {
+		void *p = NULL;
+		cudaDriverEntryPointQueryResult r;
+		if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000,
+			    cudaEnableDefault, &r) == cudaSuccess &&
+			r == cudaDriverEntryPointSuccess)
+			fn = (get_id)p;
+		cudaGetLastError();
+		__atomic_store_n(&looked, 1, __ATOMIC_RELEASE);
 	}
-	if (prec != PHASE2_PREC_FP64 && prec != PHASE2_PREC_FP32) {
-		log_error("p2d_create: unknown precision %d", prec);
-		return NULL;
+	unsigned long long id = 0;
+	if (!fn || fn(NULL, &id) != 0)
+		return 0;
+	return id;
+}
+
+static void shell_free(struct p2_dev *d)
+{
+	cudaFree(d->d_recs);
+	for (int k = 0; k < 2; k++) {
+		cudaFreeHost(d->h_recs[k]);
+		if (d->h_ev[k])
+			cudaEventDestroy(d->h_ev[k]);
 	}
+	cudaFree(d->d_idx);
+	cudaFree(d->d_val);
+	cudaFreeHost(d->h_idx);
+	cudaFreeHost(d->h_val);
+	cudaFree(d->d_part);
+	cudaFree(d->d_cm);
+	cudaFree(d->d_status);
+	cudaFreeHost(d->h_status);
+	if (d->t0)
+		cudaEventDestroy(d->t0);
+	if (d->t1)
+		cudaEventDestroy(d->t1);
+	if (d->stream)
+		cudaStreamDestroy(d->stream);
+	free(d);
+}
+
+static struct p2_dev *shell_make(int dev, uint64_t ctx)
+{
 	struct p2_dev *d = (struct p2_dev *)calloc(1, sizeof *d);
 	if (!d)
 		return NULL;
-	d->nqb = nqb;
-	d->prec = prec;
-	d->elem = prec == PHASE2_PREC_FP64 ? sizeof(double2) : sizeof(float2);
-	d->namp = UINT64_C(1) << nqb;
-	const size_t bytes = d->namp * d->elem;
-
-	int dev = 0;
-	cudaGetDevice(&dev);
+	d->device = dev;
+	d->context = ctx;
 	cudaDeviceGetAttribute(&d->sm_count, cudaDevAttrMultiProcessorCount,
 		dev);
 	if (d->sm_count <= 0)
 		d->sm_count = 148;
-	d->graphs_on = nqb <= P2_GRAPH_MAX_QB;
-
-	size_t free_b = 0, total_b = 0;
-	/* memory the pool holds but does not use can serve the state too */
-	size_t pooled = 0;
-	cudaMemPool_t pool;
-	uint64_t reserved = 0, used = 0;
-	if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
-		cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent,
-			&reserved) == cudaSuccess &&
-		cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent,
-			&used) == cudaSuccess &&
-		reserved > used)
-		pooled = (size_t)(reserved - used);
-	cudaGetLastError();
-	if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-		bytes > free_b + pooled) {
-		log_error("p2d_create: state of %zu bytes exceeds free device"
-			  " memory (%zu bytes)",
-			bytes, free_b);
-		free(d);
-		return NULL;
-	}
 	if (cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) !=
 		cudaSuccess)
 		goto fail;
-	/* stream-ordered from the default pool (p2_scratch_alloc): creating
-	 * and destroying many registers (batches) reuses memory instead of
-	 * mapping and unmapping it each time */
-	if (p2_scratch_alloc(&d->state, bytes, d->stream) != cudaSuccess) {
-		d->state = NULL;
-		log_error("p2d_create: allocation of %zu bytes failed", bytes);
-		goto fail;
-	}
 	for (int k = 0; k < 2; k++)
 		if (cudaEventCreateWithFlags(&d->h_ev[k],
 			    cudaEventDisableTiming) != cudaSuccess)
@@ -787,6 +808,137 @@ extern "C" struct p2_dev *p2d_create(uint32_t nqb, int prec)
 			d->stream) != cudaSuccess)
 		goto fail;
 	*d->h_status = 0;
+	return d;
+fail:
+	log_error("register: %s", cudaGetErrorString(cudaGetLastError()));
+	shell_free(d);
+	return NULL;
+}
+
+/* A shell of device `dev` in the current context: a kept one or a new one. */
+static struct p2_dev *shell_take(int dev)
+{
+	const uint64_t ctx = context_id();
+	struct p2_dev *d = NULL;
+	pthread_mutex_lock(&shell_lock);
+	for (int k = nshells - 1; k >= 0 && !d; k--)
+		if (shells[k]->device == dev && shells[k]->context == ctx) {
+			d = shells[k];
+			shells[k] = shells[--nshells];
+		}
+	pthread_mutex_unlock(&shell_lock);
+	return d ? d : shell_make(dev, ctx);
+}
+
+/* Keep a register's shell (its state and plans are gone) or free it. */
+static void shell_give(struct p2_dev *d)
+{
+	/* a register whose stream reports an error, or whose status word was
+	 * never read, is not reused */
+	bool keep = cudaStreamSynchronize(d->stream) == cudaSuccess &&
+		!d->status_pending;
+	const size_t held = (d->d_recs_cap + d->h_recs_cap[0] +
+				    d->h_recs_cap[1]) *
+			sizeof(struct phase2_rot_rec) +
+		d->io_cap * 48 + d->part_cap * 8 + d->cm_cap;
+	keep = keep && held <= P2_SHELL_BYTES;
+	if (keep) {
+		struct p2_dev fresh;
+		memset(&fresh, 0, sizeof fresh);
+		fresh.device = d->device;
+		fresh.context = d->context;
+		fresh.sm_count = d->sm_count;
+		fresh.stream = d->stream;
+		fresh.d_recs = d->d_recs;
+		fresh.d_recs_cap = d->d_recs_cap;
+		for (int k = 0; k < 2; k++) {
+			fresh.h_recs[k] = d->h_recs[k];
+			fresh.h_recs_cap[k] = d->h_recs_cap[k];
+			fresh.h_ev[k] = d->h_ev[k];
+		}
+		fresh.d_status = d->d_status;
+		fresh.h_status = d->h_status;
+		fresh.d_idx = d->d_idx;
+		fresh.d_val = d->d_val;
+		fresh.h_idx = d->h_idx;
+		fresh.h_val = d->h_val;
+		fresh.io_cap = d->io_cap;
+		fresh.d_part = d->d_part;
+		fresh.part_cap = d->part_cap;
+		fresh.d_cm = d->d_cm;
+		fresh.cm_cap = d->cm_cap;
+		fresh.t0 = d->t0;
+		fresh.t1 = d->t1;
+		*d = fresh;
+		pthread_mutex_lock(&shell_lock);
+		keep = nshells < P2_SHELLS;
+		if (keep)
+			shells[nshells++] = d;
+		pthread_mutex_unlock(&shell_lock);
+	}
+	if (!keep)
+		shell_free(d);
+}
+
+extern "C" void p2d_release(void)
+{
+	const uint64_t ctx = context_id();
+	pthread_mutex_lock(&shell_lock);
+	int left = 0;
+	for (int k = 0; k < nshells; k++) {
+		/* of another context: its handles are not this one's to free */
+		if (shells[k]->context == ctx)
+			shell_free(shells[k]);
+		else
+			shells[left++] = shells[k];
+	}
+	nshells = left;
+	pthread_mutex_unlock(&shell_lock);
+	int dev = 0;
+	cudaMemPool_t pool;
+	if (cudaGetDevice(&dev) == cudaSuccess &&
+		cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+		cudaMemPoolTrimTo(pool, 0);
+	cudaGetLastError();
+}
+
+extern "C" struct p2_dev *p2d_create(uint32_t nqb, int prec)
+{
+	if (nqb == 0 || nqb > 40) {
+		log_error("p2d_create: nqb=%u out of range", nqb);
+		return NULL;
+	}
+	if (prec != PHASE2_PREC_FP64 && prec != PHASE2_PREC_FP32) {
+		log_error("p2d_create: unknown precision %d", prec);
+		return NULL;
+	}
+	int dev = 0;
+	cudaGetDevice(&dev);
+	struct p2_dev *d = shell_take(dev);
+	if (!d)
+		return NULL;
+	d->nqb = nqb;
+	d->prec = prec;
+	d->elem = prec == PHASE2_PREC_FP64 ? sizeof(double2) : sizeof(float2);
+	d->namp = UINT64_C(1) << nqb;
+	const size_t bytes = d->namp * d->elem;
+	d->graphs_on = nqb <= P2_GRAPH_MAX_QB;
+
+	/* stream-ordered from the default pool (p2_scratch_alloc): creating
+	 * and destroying many registers (batches) reuses memory instead of
+	 * mapping and unmapping it each time.  The free memory is only asked
+	 * for when this fails: the query takes 0.1-0.2 ms, and on a shared
+	 * host tens of ms at times */
+	if (p2_scratch_alloc(&d->state, bytes, d->stream) != cudaSuccess) {
+		size_t free_b = 0, total_b = 0;
+		cudaGetLastError();
+		d->state = NULL;
+		(void)cudaMemGetInfo(&free_b, &total_b);
+		log_error("p2d_create: state of %zu bytes exceeds free device"
+			  " memory (%zu bytes)",
+			bytes, free_b);
+		goto fail;
+	}
 	if (cudaMemsetAsync(d->state, 0, bytes, d->stream) != cudaSuccess)
 		goto fail;
 	/* the state is ready for any stream from here on */
@@ -818,33 +970,12 @@ extern "C" void p2d_destroy(struct p2_dev *d)
 {
 	if (!d)
 		return;
-	if (d->stream)
-		cudaStreamSynchronize(d->stream);
 	if (d->state)
 		p2_scratch_free(d->state, d->stream);
-	cudaFree(d->d_recs);
-	for (int k = 0; k < 2; k++) {
-		cudaFreeHost(d->h_recs[k]);
-		if (d->h_ev[k])
-			cudaEventDestroy(d->h_ev[k]);
-	}
-	cudaFree(d->d_idx);
-	cudaFree(d->d_val);
-	cudaFreeHost(d->h_idx);
-	cudaFreeHost(d->h_val);
-	cudaFree(d->d_part);
-	cudaFree(d->d_cm);
-	cudaFree(d->d_status);
-	cudaFreeHost(d->h_status);
+	d->state = NULL;
 	for (int k = 0; k < P2_GRAPH_SLOTS; k++)
 		p2_graph_drop(d, &d->graphs[k]);
-	if (d->t0)
-		cudaEventDestroy(d->t0);
-	if (d->t1)
-		cudaEventDestroy(d->t1);
-	if (d->stream)
-		cudaStreamDestroy(d->stream);
-	free(d);
+	shell_give(d);
 }
 
 int p2_status_check(struct p2_dev *d)
@@ -1649,8 +1780,10 @@ extern "C" void *p2d_stream(const struct p2_dev *d)
 
 cudaError_t p2_scratch_alloc(void **p, size_t bytes, cudaStream_t stream)
 {
-	/* once per device (devices 0..63): keep up to 1 GiB of freed memory
-	 * in the device's default pool */
+	/* once per device (devices 0..63): keep freed memory of up to a
+	 * sixteenth of the device's in its default pool (11 GiB of 180; mapping
+	 * and unmapping a register's 8 GiB took 88 ms a run, as long as 30
+	 * passes over it); p2d_release gives it back */
 	static uint64_t pool_ready;
 	int dev = 0;
 	if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 &&
@@ -1658,6 +1791,10 @@ cudaError_t p2_scratch_alloc(void **p, size_t bytes, cudaStream_t stream)
 		cudaMemPool_t pool;
 		if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
 			uint64_t keep = UINT64_C(1) << 30;
+			size_t free_b = 0, total_b = 0;
+			if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+				total_b / 16 > keep)
+				keep = total_b / 16;
 			cudaMemPoolSetAttribute(pool,
 				cudaMemPoolAttrReleaseThreshold, &keep);
 		}

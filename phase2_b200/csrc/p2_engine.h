@@ -47,6 +47,8 @@ struct p2_dev {
 	void *state;
 	cudaStream_t stream;
 	int sm_count;
+	int device;       /* of the shell (engine.cu) */
+	uint64_t context;
 
 	struct phase2_rot_rec *d_recs;
 	size_t d_recs_cap;
@@ -113,7 +115,7 @@ static inline unsigned grid_for(const struct p2_dev *d, uint64_t work, unsigned 
 
 /* engine.cu: transient device buffers of one call (a batch program, the
  * scratch of device sampling), stream-ordered from the device's default
- * memory pool, which keeps up to 1 GiB of freed memory for the next call
+ * memory pool, which keeps up to a sixteenth of the device's memory for the next call
  * instead of unmapping it at every synchronisation (a cudaFree of such a
  * buffer could take hundreds of milliseconds).  The pool is configured on
  * the first call, for the current device (one device per process). */

@@ -59,6 +59,9 @@ void p2_tuning_at_init(void);
  * with its own non-blocking stream.  NULL on failure (logged). */
 struct p2_dev *p2d_create(uint32_t nqb, int prec);
 void p2d_destroy(struct p2_dev *d);
+/* Give back what destroyed registers left for the next ones (streams,
+ * staging, freed pool memory of the current device). */
+void p2d_release(void);
 
 int p2d_zero(struct p2_dev *d);
 int p2d_set(struct p2_dev *d, const uint64_t *idx, const double *z, size_t n);

@@ -58,8 +58,10 @@ int world_init(int *argc, char ***argv, uint64_t seed)
 
 int world_free(void)
 {
-	if (WORLD.stat == WORLD_READY)
+	if (WORLD.stat == WORLD_READY) {
 		WORLD.stat = WORLD_DONE;
+		p2d_release();
+	}
 	log_fini();
 	return WORLD.stat;
 }
