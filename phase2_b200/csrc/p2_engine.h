@@ -165,6 +165,31 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
 	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
 	uint64_t plan_id);
 
+/*
+ * resident.cu: a round of samples run on chip, one cluster each: sample s's
+ * sub-passes of chunk c are subs[s * T + c * P2_QUEUE_FLUSH ..], nsub[s * C +
+ * c] of them, records recs[s * T ..]; it starts from the determinants
+ * (widx, wval) and leaves their amplitudes in gout[s * ndet ..]; sample
+ * `keep` stores its state in the register.  nqb, lb and state are filled by
+ * the launch.
+ */
+struct p2_sub;
+struct p2_sub_rec;
+struct p2_res_samples {
+	uint32_t nqb, lb, ndet, C;
+	uint64_t T, keep;
+	const struct p2_sub *subs;
+	const uint32_t *nsub;
+	const struct p2_sub_rec *recs;
+	const uint64_t *widx;
+	const double *wval;
+	double2 *gout;
+	void *state;
+};
+bool p2_resident_samples_ok(const struct p2_dev *d, int form);
+cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
+	uint32_t g);
+
 /* lift_bulk.cu: one FP32 pass of the FP64-arithmetic form on a kernel
  * whose next cosets are staged in shared memory, by bulk copies (variant
  * 1) or cp.async (variant 2); returns 1 when launched, 0 when the pass

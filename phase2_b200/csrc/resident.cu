@@ -34,8 +34,10 @@
 #define P2_RES_MIN_QB 3
 #define P2_RES_MAX_QB 14
 #define P2_RES_TPB 256
+/* samples: many run at once, so a block may take a whole register */
+#define P2_RES_SMP_TPB 1024
 #define P2_RES_SLOTS (1 << P2_SUB_SPAN)
-#define P2_RES_SMEM (16 << 11) /* the most amplitudes of a block, 2^11 */
+#define P2_RES_SMEM (16 << 13) /* the most amplitudes of a block, 2^13 */
 
 /* ---- shared memory of the cluster --------------------------------------- */
 
@@ -140,61 +142,53 @@ __device__ __forceinline__ void p2_res_stage(uint32_t j, uint32_t nsub,
 	p2_cp_commit();
 }
 
+/* Per-block staging of k_resident's kernels. */
+struct p2_res_stagebuf {
+	struct p2_sub hdr[P2_RES_HDRS];
+	struct p2_sub_rec rec[P2_RES_STAGES][P2_SUB_ROTS];
+};
+
 /*
- * One cluster (CL) or block: blocks of 2^kc amplitudes each.  A sub-pass
- * is one trip of every amplitude through registers (8 a thread) and one
- * barrier; the records of the next sub-pass and the header after it are
+ * The sub-passes subs[0..nsub) on the register held by the cluster (CL) or
+ * block: blocks of 2^kc amplitudes each, thread t of all threads.  A
+ * sub-pass is one trip of every amplitude through registers (8 a thread)
+ * and one barrier; the records of later sub-passes and their headers are
  * copied to shared memory meanwhile.  The state is held as complex doubles
  * whatever its precision: FP32 states round at the end of each pass, where
- * the pass kernels do.
+ * the pass kernels do.  Every thread of the cluster calls it; the barrier
+ * at its start orders the caller's stores to shared memory before it.
  */
-template <typename ST, bool X, bool CL>
-__global__ void __launch_bounds__(P2_RES_TPB) k_resident(ST *__restrict__ st,
-	uint32_t nqb, uint32_t kc, const struct p2_sub *__restrict__ subs,
-	uint32_t nsub, const struct p2_sub_rec *__restrict__ recs)
+template <bool X, bool CL>
+__device__ __forceinline__ void p2_res_run(uint32_t nqb, uint32_t kc,
+	uint32_t sbase, uint32_t t, const struct p2_sub *__restrict__ subs,
+	uint32_t nsub, const struct p2_sub_rec *__restrict__ recs,
+	struct p2_res_stagebuf &sb)
 {
-	extern __shared__ __align__(16) unsigned char p2_res_dyn[];
-	__shared__ __align__(16) struct p2_sub hdr[P2_RES_HDRS];
-	__shared__ __align__(16) struct p2_sub_rec srec[P2_RES_STAGES]
-						       [P2_SUB_ROTS];
 	const uint32_t tid = threadIdx.x, nt = blockDim.x;
-	const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(p2_res_dyn);
-	const uint32_t rank = CL ? blockIdx.x : 0u;
-	const uint32_t mine = 1u << kc, first = rank << kc;
-	const uint32_t t = rank * nt + tid;
 	const bool active = t < (1u << (nqb - P2_SUB_SPAN));
-
-	/* headers of the first sub-passes (the reads of the loop below), the
-	 * block's amplitudes, then the records of the first stages */
 	for (uint32_t k = tid; k < 4 * P2_RES_HDRS && k < 4 * nsub; k += nt)
-		p2_cp16((uint32_t)__cvta_generic_to_shared(hdr) + 16 * k,
+		p2_cp16((uint32_t)__cvta_generic_to_shared(sb.hdr) + 16 * k,
 			(const unsigned char *)subs + 16 * k);
-	for (uint32_t i = tid; i < mine; i += nt) {
-		double re, im;
-		p2_ld(st, first + i, re, im);
-		p2_res_st<false>(p2_res_addr<false>(sbase,
-				 p2_sub_swz(first + i), kc), re, im);
-	}
 	p2_cp_commit();
 	p2_cp_wait<0>();
 	__syncthreads();
 	for (uint32_t j = 0; j < P2_RES_STAGES - 1; ++j)
-		p2_res_stage(j, nsub, hdr, srec, recs, tid, nt);
+		p2_res_stage(j, nsub, sb.hdr, sb.rec, recs, tid, nt);
 	p2_cp_wait<P2_RES_STAGES - 2>();
 	p2_res_barrier<CL>();
 
 	for (uint32_t i = 0; i < nsub; ++i) {
-		const struct p2_sub &h = hdr[i % P2_RES_HDRS];
-		const struct p2_sub_rec *const q0 = srec[i % P2_RES_STAGES];
+		const struct p2_sub &h = sb.hdr[i % P2_RES_HDRS];
+		const struct p2_sub_rec *const q0 = sb.rec[i % P2_RES_STAGES];
 		/* the header whose records are staged P2_RES_STAGES - 1 rounds
 		 * from now, into the place of the one just done */
 		if (i > 0 && i + P2_RES_HDRS - 1 < nsub && tid < 4)
 			p2_cp16((uint32_t)__cvta_generic_to_shared(
-					&hdr[(i - 1) % P2_RES_HDRS]) + 16 * tid,
+					&sb.hdr[(i - 1) % P2_RES_HDRS]) + 16 * tid,
 				(const unsigned char *)(subs + i +
 					P2_RES_HDRS - 1) + 16 * tid);
-		p2_res_stage(i + P2_RES_STAGES - 1, nsub, hdr, srec, recs, tid,
-			nt);
+		p2_res_stage(i + P2_RES_STAGES - 1, nsub, sb.hdr, sb.rec, recs,
+			tid, nt);
 		if (active) {
 			uint32_t x = t;
 #pragma unroll
@@ -247,12 +241,91 @@ __global__ void __launch_bounds__(P2_RES_TPB) k_resident(ST *__restrict__ st,
 		p2_res_barrier<CL>();
 	}
 	p2_cp_wait<0>();
+}
+
+/* A register's flush: load, run, store. */
+template <typename ST, bool X, bool CL>
+__global__ void __launch_bounds__(P2_RES_TPB) k_resident(ST *__restrict__ st,
+	uint32_t nqb, uint32_t kc, const struct p2_sub *__restrict__ subs,
+	uint32_t nsub, const struct p2_sub_rec *__restrict__ recs)
+{
+	extern __shared__ __align__(16) unsigned char p2_res_dyn[];
+	__shared__ __align__(16) struct p2_res_stagebuf sb;
+	const uint32_t tid = threadIdx.x, nt = blockDim.x;
+	const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(p2_res_dyn);
+	const uint32_t rank = CL ? blockIdx.x : 0u;
+	const uint32_t mine = 1u << kc, first = rank << kc;
+	for (uint32_t i = tid; i < mine; i += nt) {
+		double re, im;
+		p2_ld(st, first + i, re, im);
+		p2_res_st<false>(p2_res_addr<false>(sbase,
+				 p2_sub_swz(first + i), kc), re, im);
+	}
+	p2_res_run<X, CL>(nqb, kc, sbase, rank * nt + tid, subs, nsub, recs, sb);
 	for (uint32_t i = tid; i < mine; i += nt) {
 		double re, im;
 		p2_res_ld<false>(p2_res_addr<false>(sbase,
 				 p2_sub_swz(first + i), kc), re, im);
 		p2_st(st, first + i, re, im);
 	}
+}
+
+/*
+ * Samples of a sampled driver (sampling.cu), one cluster of 2^lb blocks
+ * each, entirely on chip: zero, the trial state's determinants (in order:
+ * later writes win), the sub-passes of every chunk, the determinants'
+ * amplitudes out.  Only sample `keep` of the round stores its state.
+ */
+template <typename ST, bool X, bool CL>
+__global__ void __launch_bounds__(P2_RES_SMP_TPB) k_resident_smp(
+	const struct p2_res_samples a)
+{
+	extern __shared__ __align__(16) unsigned char p2_res_dyn[];
+	__shared__ __align__(16) struct p2_res_stagebuf sb;
+	const uint32_t tid = threadIdx.x, nt = blockDim.x;
+	const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(p2_res_dyn);
+	const uint32_t kc = a.nqb - a.lb, low = (1u << kc) - 1u;
+	const uint64_t s = blockIdx.x >> a.lb;
+	const uint32_t rank = CL ? blockIdx.x & ((1u << a.lb) - 1u) : 0u;
+	const uint32_t mine = 1u << kc, first = rank << kc;
+	for (uint32_t i = tid; i < mine; i += nt)
+		p2_res_st<false>(sbase + 16 * i, 0.0, 0.0);
+	__syncthreads();
+	if (tid == 0)
+		for (uint32_t e = 0; e < a.ndet; ++e) {
+			const uint32_t g = (uint32_t)a.widx[e];
+			if (g >> kc != rank)
+				continue;
+			double re = a.wval[2 * e], im = a.wval[2 * e + 1];
+			if (sizeof(ST) == 8) {
+				re = (double)__double2float_rn(re);
+				im = (double)__double2float_rn(im);
+			}
+			p2_res_st<false>(sbase + 16 * (p2_sub_swz(g) & low), re,
+				im);
+		}
+	const struct p2_sub_rec *const recs = a.recs + s * a.T;
+	for (uint32_t c = 0; c < a.C; ++c)
+		p2_res_run<X, CL>(a.nqb, kc, sbase, rank * nt + tid,
+			a.subs + s * a.T + (uint64_t)c * P2_QUEUE_FLUSH,
+			a.nsub[s * a.C + c], recs, sb);
+	/* its last barrier (or, without sub-passes, its first) ordered every
+	 * block's stores before these reads of the block's own part */
+	for (uint32_t e = tid; e < a.ndet; e += nt) {
+		const uint32_t g = (uint32_t)a.widx[e];
+		if (g >> kc != rank)
+			continue;
+		double re, im;
+		p2_res_ld<false>(sbase + 16 * (p2_sub_swz(g) & low), re, im);
+		a.gout[s * a.ndet + e] = make_double2(re, im);
+	}
+	if (s == a.keep)
+		for (uint32_t i = tid; i < mine; i += nt) {
+			double re, im;
+			p2_res_ld<false>(sbase + 16 *
+					(p2_sub_swz(first + i) & low), re, im);
+			p2_st((ST *)a.state, first + i, re, im);
+		}
 }
 
 /* ---- host side ----------------------------------------------------------- */
@@ -395,28 +468,28 @@ fail:
 	return NULL;
 }
 
-/* Largest cluster the kernel can be launched with on this device (blocks of
- * 128 threads and 16 KiB), once per instantiation; 0 when it cannot be
+/* Largest cluster a kernel can be launched with on this device (blocks of
+ * 128 threads and 16 KiB), once per kernel; 0 when it cannot be
  * configured. */
-template <typename ST, bool X, bool CL> static unsigned res_clusters(void)
+template <auto F> static unsigned res_clusters(bool clusters)
 {
 	static unsigned most; /* 1 + the answer */
 	unsigned m = __atomic_load_n(&most, __ATOMIC_ACQUIRE);
 	if (m)
 		return m - 1;
 	unsigned best = 0;
-	if (cudaFuncSetAttribute(k_resident<ST, X, CL>,
-		    cudaFuncAttributeMaxDynamicSharedMemorySize,
+	if (cudaFuncSetAttribute(F, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		    P2_RES_SMEM) == cudaSuccess) {
 		best = 1;
-		if (CL && cudaFuncSetAttribute(k_resident<ST, X, CL>,
-				  cudaFuncAttributeNonPortableClusterSizeAllowed,
-				  1) != cudaSuccess)
+		if (clusters && cudaFuncSetAttribute(F,
+				cudaFuncAttributeNonPortableClusterSizeAllowed,
+				1) != cudaSuccess)
 			best = 0;
-		for (unsigned c = 16; CL && best == 1 && c > 1; c /= 2) {
+		for (unsigned c = 16; clusters && best == 1 && c > 1; c /= 2) {
 			cudaLaunchConfig_t cfg;
 			cudaLaunchAttribute at[1];
 			memset(&cfg, 0, sizeof cfg);
+			memset(at, 0, sizeof at);
 			at[0].id = cudaLaunchAttributeClusterDimension;
 			at[0].val.clusterDim.x = c;
 			at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -426,8 +499,7 @@ template <typename ST, bool X, bool CL> static unsigned res_clusters(void)
 			cfg.attrs = at;
 			cfg.numAttrs = 1;
 			int n = 0;
-			if (cudaOccupancyMaxActiveClusters(&n,
-				    k_resident<ST, X, CL>, &cfg) ==
+			if (cudaOccupancyMaxActiveClusters(&n, F, &cfg) ==
 					cudaSuccess && n > 0)
 				best = c;
 		}
@@ -437,46 +509,63 @@ template <typename ST, bool X, bool CL> static unsigned res_clusters(void)
 	return best;
 }
 
+/* A register width and form the kernels here take. */
+static bool res_width_ok(const struct p2_dev *d, int form)
+{
+	return d->nqb >= P2_RES_MIN_QB && d->nqb <= P2_RES_MAX_QB &&
+		form != PHASE2_FORM_LIFTED_F32;
+}
+
 bool p2_resident_ok(const struct p2_dev *d, int form)
 {
-	if (d->nqb < P2_RES_MIN_QB || d->nqb > P2_RES_MAX_QB ||
-		form == PHASE2_FORM_LIFTED_F32)
+	if (!res_width_ok(d, form))
 		return false;
 	const uint32_t lb = res_log_blocks(d->nqb);
 	const unsigned most = d->prec == PHASE2_PREC_FP64
-		? (lb ? res_clusters<double2, false, true>()
-		      : res_clusters<double2, false, false>())
-		: (lb ? res_clusters<float2, true, true>()
-		      : res_clusters<float2, true, false>());
+		? (lb ? res_clusters<k_resident<double2, false, true>>(true)
+		      : res_clusters<k_resident<double2, false, false>>(false))
+		: (lb ? res_clusters<k_resident<float2, true, true>>(true)
+		      : res_clusters<k_resident<float2, true, false>>(false));
 	return most >= (1u << lb);
 }
 
-template <typename ST, bool X, bool CL>
-static int res_launch(struct p2_dev *d, uint32_t lb, const struct p2_graph *g)
+/* Launch blocks of a register's (or sample's) share in clusters of 2^lb:
+ * grid blocks, one thread for 8 amplitudes. */
+template <typename F, typename... A>
+static cudaError_t res_launch(F *fn, unsigned grid, uint32_t nqb, uint32_t lb,
+	cudaStream_t stream, A... args)
 {
-	const uint32_t kc = d->nqb - lb;
-	const size_t smem = (size_t)16 << kc;
-	uint32_t tpb = 1u << (d->nqb - P2_SUB_SPAN - lb);
-	if (tpb < 32)
-		tpb = 32;
 	cudaLaunchConfig_t cfg;
 	cudaLaunchAttribute at[1];
+	uint32_t tpb = 1u << (nqb - P2_SUB_SPAN - lb);
+	if (tpb < 32)
+		tpb = 32;
 	memset(&cfg, 0, sizeof cfg);
-	cfg.gridDim = dim3(1u << lb);
+	memset(at, 0, sizeof at);
+	cfg.gridDim = dim3(grid);
 	cfg.blockDim = dim3(tpb);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = d->stream;
-	if (CL) {
+	cfg.dynamicSmemBytes = (size_t)16 << (nqb - lb);
+	cfg.stream = stream;
+	if (lb) {
 		at[0].id = cudaLaunchAttributeClusterDimension;
 		at[0].val.clusterDim.x = 1u << lb;
 		at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
 		cfg.attrs = at;
 		cfg.numAttrs = 1;
 	}
+	return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+template <typename ST, bool X>
+static int res_launch_flush(struct p2_dev *d, const struct p2_graph *g)
+{
+	const uint32_t lb = res_log_blocks(d->nqb);
 	const struct p2_sub_rec *sr = (const struct p2_sub_rec *)g->d_recs;
-	CUDA_OK(cudaLaunchKernelEx(&cfg, k_resident<ST, X, CL>, (ST *)d->state,
-			d->nqb, kc, (const struct p2_sub *)(sr + g->nrec),
-			g->nsub, sr),
+	const struct p2_sub *subs = (const struct p2_sub *)(sr + g->nrec);
+	CUDA_OK(res_launch(lb ? k_resident<ST, X, true>
+			      : k_resident<ST, X, false>,
+			1u << lb, d->nqb, lb, d->stream, (ST *)d->state, d->nqb,
+			d->nqb - lb, subs, g->nsub, sr),
 		"resident launch");
 	return 0;
 }
@@ -491,15 +580,63 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
 	if (!g)
 		return -1;
 	d->graph_replays += hit;
-	const uint32_t lb = res_log_blocks(d->nqb);
 	if (d->timing)
 		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
-	int rc;
-	if (d->prec == PHASE2_PREC_FP64)
-		rc = lb ? res_launch<double2, false, true>(d, lb, g)
-			: res_launch<double2, false, false>(d, lb, g);
-	else
-		rc = lb ? res_launch<float2, true, true>(d, lb, g)
-			: res_launch<float2, true, false>(d, lb, g);
-	return rc;
+	return d->prec == PHASE2_PREC_FP64
+		? res_launch_flush<double2, false>(d, g)
+		: res_launch_flush<float2, true>(d, g);
+}
+
+/* ---- samples -------------------------------------------------------------- */
+
+/*
+ * log2 of a sample's blocks in a round of g samples: more blocks shorten one
+ * sample, but the traffic between them costs throughput, so only as many as
+ * leave half of the SMs a block (1000 draws, us a call, blocks a sample 1 /
+ * 2 / 4 / 8 / 16: 13 qubits, 8 samples 1534 / 1441 / 1353 / 1118 / 1150, 32
+ * samples 1581 / 1512 / 1485 / 1577 / 1724, 128 samples 1812 / 2424 / 3651 /
+ * 3964 / 4559).  A block holds 2^13 amplitudes at most.
+ */
+static uint32_t res_sample_blocks(const struct p2_dev *d, uint64_t g)
+{
+	const uint32_t least = d->nqb > 13 ? d->nqb - 13 : 0;
+	uint32_t lb = res_log_blocks(d->nqb);
+	while (lb > least && (g << lb) > (uint64_t)d->sm_count / 2)
+		lb--;
+	return lb;
+}
+
+bool p2_resident_samples_ok(const struct p2_dev *d, int form)
+{
+	if (!res_width_ok(d, form))
+		return false;
+	const uint32_t lb = res_log_blocks(d->nqb);
+	const unsigned most = d->prec == PHASE2_PREC_FP64
+		? (lb ? res_clusters<k_resident_smp<double2, false, true>>(true)
+		      : res_clusters<k_resident_smp<double2, false, false>>(
+				false))
+		: (lb ? res_clusters<k_resident_smp<float2, true, true>>(true)
+		      : res_clusters<k_resident_smp<float2, true, false>>(
+				false));
+	return most >= (1u << lb);
+}
+
+template <typename ST, bool X>
+static cudaError_t res_launch_samples(struct p2_dev *d,
+	const struct p2_res_samples &a, uint32_t g)
+{
+	return res_launch(a.lb ? k_resident_smp<ST, X, true>
+			       : k_resident_smp<ST, X, false>,
+		g << a.lb, a.nqb, a.lb, d->stream, a);
+}
+
+cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
+	uint32_t g)
+{
+	a.nqb = d->nqb;
+	a.lb = res_sample_blocks(d, g);
+	a.state = d->state;
+	return d->prec == PHASE2_PREC_FP64
+		? res_launch_samples<double2, false>(d, a, g)
+		: res_launch_samples<float2, true>(d, a, g);
 }

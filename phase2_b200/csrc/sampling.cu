@@ -18,6 +18,7 @@
 
 #include "p2_kernels.cuh"
 #include "plan_core.h"
+#include "sub_core.h"
 
 /* ---- device-side qDRIFT ------------------------------------------------- */
 
@@ -228,7 +229,9 @@ __global__ void __launch_bounds__(P2_SMP_PLAN_TPB)
 	k_smp_plan(const struct p2_smp_job job, uint64_t T, uint32_t C,
 		const struct phase2_rot_in *__restrict__ rot,
 		const double *__restrict__ cs, struct phase2_pass *passes,
-		struct phase2_rot_rec *__restrict__ recs, uint32_t *npc)
+		struct phase2_rot_rec *__restrict__ recs, uint32_t *npc,
+		struct p2_sub *__restrict__ tmp, struct p2_sub *__restrict__ subs,
+		struct p2_sub_rec *__restrict__ srec, uint32_t *nsub)
 {
 	extern __shared__ __align__(16) unsigned char sm[];
 	uint64_t *fl = (uint64_t *)sm;
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(P2_SMP_PLAN_TPB)
 	uint8_t *U = (uint8_t *)(pid + P2_QUEUE_FLUSH);
 	uint32_t *neg = (uint32_t *)(U + P2_QUEUE_FLUSH);
 	__shared__ long s_np;
+	__shared__ uint32_t part[P2_SMP_PLAN_TPB];
 	const uint64_t s = blockIdx.x / C, c = blockIdx.x - s * C;
 	const uint64_t at = s * T + c * P2_QUEUE_FLUSH;
 	const uint32_t n = (uint32_t)(T - c * P2_QUEUE_FLUSH < P2_QUEUE_FLUSH
@@ -273,8 +277,11 @@ __global__ void __launch_bounds__(P2_SMP_PLAN_TPB)
 		__syncthreads();
 	}
 	if (np < 0) {
-		if (threadIdx.x == 0)
+		if (threadIdx.x == 0) {
 			npc[blockIdx.x] = 0;
+			if (subs)
+				nsub[blockIdx.x] = 0;
+		}
 		return;
 	}
 	for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -292,6 +299,39 @@ __global__ void __launch_bounds__(P2_SMP_PLAN_TPB)
 	}
 	if (threadIdx.x == 0)
 		npc[blockIdx.x] = (uint32_t)np;
+	if (!subs)
+		return;
+	/* samples run on chip: each pass's sub-passes, at the places of its
+	 * rotations first, then moved together in pass order (pid holds the
+	 * counts; each thread takes consecutive passes) */
+	__syncthreads();
+	const uint32_t per = ((uint32_t)np + blockDim.x - 1) / blockDim.x;
+	const uint32_t p0 = threadIdx.x * per < (uint32_t)np
+		? threadIdx.x * per : (uint32_t)np;
+	const uint32_t p1 = p0 + per < (uint32_t)np ? p0 + per : (uint32_t)np;
+	uint32_t mine = 0;
+	for (uint32_t p = p0; p < p1; ++p) {
+		const uint32_t off = passes[at + p].rot_off;
+		const uint32_t k = p2_sub_split(&passes[at + p], recs + off,
+			job.nqb, off - (uint32_t)(s * T), tmp + off, srec + off);
+		pid[p] = (uint16_t)k;
+		mine += k;
+	}
+	part[threadIdx.x] = mine;
+	__syncthreads();
+	uint32_t base = 0, all = 0;
+	for (uint32_t k = 0; k < blockDim.x; ++k) {
+		base += k < threadIdx.x ? part[k] : 0u;
+		all += part[k];
+	}
+	for (uint32_t p = p0; p < p1; ++p) {
+		const uint32_t off = passes[at + p].rot_off;
+		for (uint32_t k = 0; k < pid[p]; ++k)
+			subs[at + base + k] = tmp[off + k];
+		base += pid[p];
+	}
+	if (threadIdx.x == 0)
+		nsub[blockIdx.x] = all;
 }
 
 /*
@@ -375,6 +415,23 @@ __global__ void k_smp_fill(const struct p2_smp_job job, uint32_t g,
 	}
 }
 
+/* Stage times of a round on stderr (PHASE2_SAMPLING_TIMING=1). */
+static void smp_report(const cudaEvent_t *ev, uint32_t g, uint64_t T,
+	uint32_t nreg, uint64_t ops, unsigned grid)
+{
+	float t[4];
+	for (int i = 0; i < 4; i++)
+		cudaEventElapsedTime(&t[i], ev[i], ev[i + 1]);
+	fprintf(stderr,
+		"device sampling: %u samples x %llu rotations, %u registers,"
+		" %llu ops, grid %u: draw+stream %.3f ms, plan %.3f ms, layout"
+		" %.3f ms, run %.3f ms\n",
+		g, (unsigned long long)T, nreg, (unsigned long long)ops, grid,
+		t[0], t[1], t[2], t[3]);
+}
+
+/* Tables of a run copied through the register's pinned staging at most. */
+#define P2_SMP_STAGE ((size_t)1 << 20)
 /* Rotations held per device round (rotation scratch, plans, program). */
 #define P2_SMP_ROUND_ROTS (UINT64_C(1) << 21)
 /* Amplitudes of all the registers of one round together (FP32: 512 MiB);
@@ -414,10 +471,19 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 	if (R < 1)
 		R = 1;
 	const uint32_t C = (uint32_t)((T + P2_QUEUE_FLUSH - 1) / P2_QUEUE_FLUSH);
+	/* registers that fit on chip: no state copies, no persistent kernel */
+	const bool res = T > 0 && p2_resident_samples_ok(d, job->form);
+	if (res) {
+		R = 1;
+		/* twice the scratch a rotation */
+		if (G > 1 && G * T > P2_SMP_ROUND_ROTS / 2)
+			G = (G + 1) / 2;
+	}
 	const size_t nt = job->nterms, nd = job->ndet, nh = job->length;
 	/* device buffer: tables, per-round scratch and program, registers */
 	enum { RNG, CDF, TFL, TPH, TCF, HFL, HPH, HPHI, HCS, WIDX, WVAL, GIDX,
-		GOUT, X, ROT, CS, PASS, REC, PROG, NPC, SOFF, POFF, REGS, NBUF };
+		GOUT, X, ROT, CS, PASS, REC, PROG, NPC, SOFF, POFF, REGS, SUBT,
+		SUB, SREC, NSUB, NBUF };
 	size_t sz[NBUF], off[NBUF], total = 0;
 	/* sizes and offsets for rounds of G samples on R registers */
 	auto layout = [&](size_t G, size_t R) {
@@ -441,6 +507,11 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		sz[PROG] = (G * T + 3 * G) * sizeof(struct p2_op);
 		sz[NPC] = sz[POFF] = (G * C != 0 ? G * C : 1) * sizeof(uint32_t);
 		sz[SOFF] = G * sizeof(uint32_t);
+		sz[SUBT] = sz[SUB] = res ? GT * sizeof(struct p2_sub) : 0;
+		sz[SREC] = res ? GT * sizeof(struct p2_sub_rec) : 0;
+		sz[NSUB] = res ? sz[NPC] : 0;
+		if (res)
+			sz[PROG] = sz[GIDX] = 0;
 		sz[REGS] = R * (sizeof(struct p2_binst) +
 				       sizeof(struct p2_bctl)) +
 			4 * sizeof(unsigned int) + (R - 1) * d->namp * d->elem;
@@ -471,11 +542,12 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		}
 	}
 	uint64_t *gidx = (uint64_t *)malloc(sz[GIDX] ? sz[GIDX] : 1);
+	uint32_t *hnpc = (uint32_t *)malloc(sz[NPC]);
 	struct p2_binst *hinst = (struct p2_binst *)malloc(
 		R * sizeof(struct p2_binst));
 	int rc = -1;
-	cudaError_t e = gidx && hinst ? cudaSuccess
-				      : cudaErrorMemoryAllocation;
+	cudaError_t e = gidx && hinst && hnpc ? cudaSuccess
+					      : cudaErrorMemoryAllocation;
 	/* registers: the copies first (256-aligned), then inst, ctl, status */
 	unsigned char *copies = b + off[REGS];
 	struct p2_binst *inst = (struct p2_binst *)(b + off[REGS] +
@@ -483,7 +555,7 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 	struct p2_bctl *ctl = (struct p2_bctl *)(inst + R);
 	unsigned int *status = (unsigned int *)(ctl + R);
 	if (e == cudaSuccess) {
-		for (size_t s = 0; s < samples; s++)
+		for (size_t s = 0; s < samples && !res; s++)
 			for (size_t j = 0; j < nd; j++)
 				gidx[s * nd + j] = det_idx[j];
 		for (size_t r = 0; r < R; r++) {
@@ -497,21 +569,36 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 			hphase, hphi, hcs, det_idx, det_val, gidx };
 		const int at[] = { RNG, CDF, TFL, TPH, TCF, HFL, HPH, HPHI, HCS,
 			WIDX, WVAL, GIDX };
-		for (int i = 0; i < 12 && e == cudaSuccess; i++)
+		/* the tables are the buffer's first part: one copy through the
+		 * pinned staging unless they are large */
+		const size_t tables = off[GIDX] + sz[GIDX];
+		const bool once = tables <= P2_SMP_STAGE;
+		if (once) {
+			unsigned char *h = (unsigned char *)p2_stage_reserve(d,
+				(tables + 31) / 32);
+			if (!h)
+				e = cudaErrorMemoryAllocation;
+			for (int i = 0; h && i < 12; i++)
+				if (sz[at[i]])
+					memcpy(h + off[at[i]], src[i], sz[at[i]]);
+			if (h && p2_stage_upload(d, b, tables) < 0)
+				e = cudaErrorUnknown;
+		}
+		for (int i = 0; i < 12 && e == cudaSuccess && !once; i++)
 			if (sz[at[i]]) {
 				e = cudaMemcpyAsync(b + off[at[i]], src[i],
 					sz[at[i]], cudaMemcpyHostToDevice,
 					d->stream);
 				d->h2d_bytes += sz[at[i]];
 			}
-		if (e == cudaSuccess)
+		if (e == cudaSuccess && !res)
 			e = cudaMemcpyAsync(inst, hinst,
 				R * sizeof(struct p2_binst),
 				cudaMemcpyHostToDevice, d->stream);
 	}
 	const int kind = p2_batch_kind(d->prec, job->form);
 	int per_sm = 0;
-	if (e == cudaSuccess)
+	if (e == cudaSuccess && !res)
 		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
 			p2_batch_kernel(kind), P2_TPB, 0);
 	if (e == cudaSuccess)
@@ -575,9 +662,50 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 				(const struct phase2_rot_in *)(b + off[ROT]),
 				(const double *)(b + off[CS]),
 				(struct phase2_pass *)(b + off[PASS]),
-				(struct phase2_rot_rec *)(b + off[REC]), npc);
+				(struct phase2_rot_rec *)(b + off[REC]), npc,
+				(struct p2_sub *)(b + off[SUBT]),
+				res ? (struct p2_sub *)(b + off[SUB]) : NULL,
+				(struct p2_sub_rec *)(b + off[SREC]),
+				(uint32_t *)(b + off[NSUB]));
 		if (timing)
 			cudaEventRecord(ev[2], d->stream);
+		if (res) {
+			struct p2_res_samples a;
+			memset(&a, 0, sizeof a);
+			a.ndet = job->ndet;
+			a.C = C;
+			a.T = T;
+			/* the run's last sample ends in the register */
+			a.keep = s0 + g == samples ? g - 1 : UINT64_MAX;
+			a.subs = (const struct p2_sub *)(b + off[SUB]);
+			a.nsub = (const uint32_t *)(b + off[NSUB]);
+			a.recs = (const struct p2_sub_rec *)(b + off[SREC]);
+			a.widx = (const uint64_t *)(b + off[WIDX]);
+			a.wval = (const double *)(b + off[WVAL]);
+			a.gout = (double2 *)(b + off[GOUT]) + s0 * job->ndet;
+			e = cudaGetLastError();
+			if (timing)
+				cudaEventRecord(ev[3], d->stream);
+			if (e == cudaSuccess)
+				e = p2_resident_samples(d, a, g);
+			if (timing)
+				cudaEventRecord(ev[4], d->stream);
+			d->launches += 3 + (job->depth != 0);
+			if (e == cudaSuccess)
+				e = cudaMemcpyAsync(hnpc, npc,
+					(size_t)g * C * sizeof *hnpc,
+					cudaMemcpyDeviceToHost, d->stream);
+			if (e == cudaSuccess)
+				e = cudaStreamSynchronize(d->stream);
+			uint64_t np = 0;
+			for (size_t k = 0; e == cudaSuccess && k < (size_t)g * C;
+				k++)
+				np += hnpc[k];
+			nops_run += np;
+			if (timing && e == cudaSuccess)
+				smp_report(ev, g, T, g, np + 3ull * g, 0);
+			continue;
+		}
 		k_smp_layout<<<1, 32, 0, d->stream>>>(g, C, npc,
 			(uint64_t)samples - 1, (uint64_t)s0, nreg, soff, poff,
 			inst);
@@ -629,19 +757,8 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		for (uint32_t r = 0; e == cudaSuccess && r < nreg; r++)
 			rops += hinst[r].nops;
 		nops_run += rops - 3ull * g;
-		if (timing && e == cudaSuccess) {
-			float t[4];
-			for (int i = 0; i < 4; i++)
-				cudaEventElapsedTime(&t[i], ev[i], ev[i + 1]);
-			fprintf(stderr,
-				"device sampling: %u samples x %llu rotations,"
-				" %u registers, %llu ops, grid %u: draw+stream"
-				" %.3f ms, plan %.3f ms, layout %.3f ms, run"
-				" %.3f ms\n",
-				g, (unsigned long long)T, nreg,
-				(unsigned long long)rops, grid, t[0], t[1], t[2],
-				t[3]);
-		}
+		if (timing && e == cudaSuccess)
+			smp_report(ev, g, T, nreg, rops, grid);
 	}
 	for (int i = 0; timing && i < 5; i++)
 		cudaEventDestroy(ev[i]);
@@ -660,6 +777,7 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 	}
 	free(gidx);
 	free(hinst);
+	free(hnpc);
 	p2_scratch_free(b, d->stream);
 	return rc;
 }
