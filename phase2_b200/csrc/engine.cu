@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(p2_tpb(M), p2_min_blocks(M))
 			sbasis[k] = p.basis[k];
 	}
 	__syncthreads();
+	p2_grid_wait();
 	uint64_t pb[M > 0 ? M : 1];
 #pragma unroll
 	for (int k = 0; k < M; ++k)
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(P2_TPB, p2_min_blocks(M))
 			sbasis[k] = p.basis[k];
 	}
 	__syncthreads();
+	p2_grid_wait();
 	uint64_t pb[M > 0 ? M : 1];
 #pragma unroll
 	for (int k = 0; k < M; ++k)
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(P2_TPB, M >= 5 ? 3 : p2_min_blocks(M))
 		srec[r] = o;
 	}
 	__syncthreads();
+	p2_grid_wait();
 	IT pb[M > 0 ? M : 1];
 #pragma unroll
 	for (int k = 0; k < M; ++k)
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 	for (uint32_t r = threadIdx.x; r < p.nrot; r += blockDim.x)
 		srec[r] = p2_lift32_of(recs[p.rot_off + r]);
 	__syncthreads();
+	p2_grid_wait();
 	IT pb[M > 0 ? M : 1];
 #pragma unroll
 	for (int k = 0; k < M; ++k)
@@ -267,13 +271,6 @@ __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
  * the start of the pass.  Below it, the absolute error of an FP32 shear
  * (half an ulp) is at most 2^-35. */
 #define P2_HEAVY_MIN 0x1p-10f
-
-/* Registers below this many qubits run mixed-form passes on the FP64-
- * arithmetic kernels: a spread state of n qubits has components of
- * standard deviation 2^-(n+1)/2, which reach P2_HEAVY_MIN often below 24
- * qubits (at 22, a quarter of the cosets), and a heavy coset costs its
- * warp a serial FP64 run; at 24 the threshold is 5.7 deviations away. */
-#define P2_MIXED_MIN_QB 24
 
 /*
  * The run of rotations on one coset held in shared memory as FP64 (hv: 2^M
@@ -364,6 +361,7 @@ __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 		tt[r] = recs[p.rot_off + r].c;
 	}
 	__syncthreads();
+	p2_grid_wait();
 	IT pb[M > 0 ? M : 1];
 #pragma unroll
 	for (int k = 0; k < M; ++k)
@@ -963,6 +961,7 @@ void p2_graph_drop(struct p2_dev *d, struct p2_graph *g)
 	}
 	free(g->passes);
 	free(g->recs);
+	free(g->split);
 	memset(g, 0, sizeof *g);
 }
 
@@ -1211,7 +1210,9 @@ static int launch_pass_t(struct p2_dev *d, const struct phase2_pass &p,
 	if (te.variant != 1) {
 		const unsigned per_sm = te.per_sm ? (unsigned)te.per_sm : 16u;
 		const unsigned grid = grid_for(d, nrep, P2_TPB, per_sm);
-		k_pass<M><<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+		CUDA_OK(p2_launch(k_pass<M>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 		return 0;
 	}
 	static struct p2_kcfg cfg;
@@ -1233,7 +1234,9 @@ static int launch_pass_t(struct p2_dev *d, const struct phase2_pass &p,
 		? (unsigned)te.per_sm
 		: (unsigned)cfg.per_sm;
 	const unsigned grid = grid_for(d, nrep, (unsigned)cfg.tpb, per_sm);
-	k_pass_pf<M><<<grid, cfg.tpb, cfg.smem, d->stream>>>(sv, nrep, p, recs);
+	CUDA_OK(p2_launch(k_pass_pf<M>, grid, cfg.tpb, cfg.smem,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 	return 0;
 }
 
@@ -1252,19 +1255,23 @@ static int launch_lift_t(struct p2_dev *d, const struct phase2_pass &p,
 	const bool narrow = d->nqb <= 31;
 	if (p.form == PHASE2_FORM_LIFTED_F32) {
 		if (narrow)
-			k_pass_lift32<M, uint32_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift32<M, uint32_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 		else
-			k_pass_lift32<M, uint64_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift32<M, uint64_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 	} else if (p.form == PHASE2_FORM_LIFTED_MIXED &&
 		d->nqb >= P2_MIXED_MIN_QB) {
 		if (narrow)
-			k_pass_lift32h<M, uint32_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift32h<M, uint32_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 		else
-			k_pass_lift32h<M, uint64_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift32h<M, uint64_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 	} else if (p.form == PHASE2_FORM_LIFTED ||
 		p.form == PHASE2_FORM_LIFTED_MIXED) {
 		/* mixed-form passes of smaller registers: FP64 arithmetic on
@@ -1279,11 +1286,13 @@ static int launch_lift_t(struct p2_dev *d, const struct phase2_pass &p,
 				return rc < 0 ? -1 : 0;
 		}
 		if (narrow)
-			k_pass_lift<M, uint32_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift<M, uint32_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 		else
-			k_pass_lift<M, uint64_t>
-				<<<grid, P2_TPB, 0, d->stream>>>(sv, nrep, p, recs);
+			CUDA_OK(p2_launch(k_pass_lift<M, uint64_t>, grid, P2_TPB, 0,
+				d->stream, sv, nrep, p, recs),
+			"pass launch");
 	} else {
 		log_error("FP32 pass of form %u unsupported", p.form);
 		return -1;
@@ -1502,7 +1511,8 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 {
 	if (npass == 0)
 		return 0;
-	const bool resident = p2_resident_ok(d, passes[0].form);
+	const bool split = p2_split_ok(d, passes[0].form);
+	const bool resident = split || p2_resident_ok(d, passes[0].form);
 	struct p2_graph *g = resident
 		? NULL
 		: graph_for(d, passes, npass, recs, nrec);
@@ -1522,9 +1532,10 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	long launches;
 	if (resident) {
 		/* counted as one state round trip a pass, as planned */
-		if (p2_resident_run(d, passes, npass, recs, nrec, plan_id) < 0)
+		if ((split ? p2_split_run : p2_resident_run)(d, passes, npass,
+			    recs, nrec, plan_id) < 0)
 			return -1;
-		d->launches++;
+		d->launches += split ? npass : 1;
 		launches = (long)npass;
 	} else if (g) {
 		CUDA_OK(cudaGraphLaunch(g->exec, d->stream), "graph launch");

@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(P2_LB_TPB, MINB)
 		srec[r] = o;
 	}
 	__syncthreads();
+	p2_grid_wait();
 
 	const uint32_t dyn = p2_saddr(p2_lb_dyn);
 	const uint32_t pad = ((dyn + 255u) & ~255u) - dyn;
@@ -408,9 +409,10 @@ static int pf_launch_t(struct p2_dev *d, const struct phase2_pass *p,
 		cfg.ready = 1;
 	}
 	const uint32_t nwc = (uint32_t)((d->namp >> M) >> 5);
-	k_pass_lift_pf<M, MINB><<<lb_grid(d, cfg.per_sm, per_sm_cap, nwc),
-		P2_LB_TPB, smem, d->stream>>>((float2 *)d->state, nwc, *p,
-		recs);
+	CUDA_OK(p2_launch(k_pass_lift_pf<M, MINB>,
+			lb_grid(d, cfg.per_sm, per_sm_cap, nwc), P2_LB_TPB, smem,
+			d->stream, (float2 *)d->state, nwc, *p, recs),
+		"staged pass launch");
 	return 1;
 }
 

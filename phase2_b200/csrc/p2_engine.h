@@ -9,12 +9,20 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "phase2_b200.h"
 
 #include "p2_internal.h"
 
 #define P2_TPB 128
+
+/* Registers below this many qubits run mixed-form passes on the FP64-
+ * arithmetic kernels: a spread state of n qubits has components of
+ * standard deviation 2^-(n+1)/2, which reach P2_HEAVY_MIN often below 24
+ * qubits (at 22, a quarter of the cosets), and a heavy coset costs its
+ * warp a serial FP64 run; at 24 the threshold is 5.7 deviations away. */
+#define P2_MIXED_MIN_QB 24
 #define P2_RED_TPB 256
 
 /* Replay of repeated flushes: registers up to this width keep a small LRU
@@ -34,6 +42,7 @@ struct p2_graph {
 	 * records and its nsub sub-passes, d_cap bytes from the pool */
 	size_t d_cap;
 	uint32_t nsub;
+	struct p2_split_pass *split; /* per pass (split.cu), or NULL */
 	uint64_t plan_id; /* the caller's number of this plan (0: none) */
 	int status;     /* the graph holds kernels that write d_status */
 	uint64_t used;
@@ -111,6 +120,40 @@ static inline unsigned grid_for(const struct p2_dev *d, uint64_t work, unsigned 
 	return b ? (unsigned)b : 1u;
 }
 
+#ifdef __CUDACC__
+/*
+ * A pass kernel's launch: it may start before the previous kernel of the
+ * stream has ended (programmatic dependent launch), stages its records, and
+ * waits (p2_grid_wait) before it touches the state.  A pass of a register
+ * that fits the L2 cache takes 3-10 us, of which the launch gap was 2-3.
+ * Records are uploaded by copies, which such a launch still waits for.
+ */
+template <typename... P, typename... A>
+static cudaError_t p2_launch(void (*fn)(P...), unsigned grid, unsigned tpb,
+	size_t smem, cudaStream_t stream, A... args)
+{
+	cudaLaunchConfig_t cfg;
+	cudaLaunchAttribute at[1];
+	memset(&cfg, 0, sizeof cfg);
+	memset(at, 0, sizeof at);
+	cfg.gridDim = dim3(grid);
+	cfg.blockDim = dim3(tpb);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = stream;
+	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+
+/* Wait for the previous kernel's end and its stores. */
+__device__ __forceinline__ void p2_grid_wait()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 /* ---- cross-file entry points -------------------------------------------- */
 
 /* engine.cu: transient device buffers of one call (a batch program, the
@@ -162,6 +205,21 @@ void p2_graph_drop(struct p2_dev *d, struct p2_graph *g);
  * flushes with the same passes and records. */
 bool p2_resident_ok(const struct p2_dev *d, int form);
 int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
+	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
+	uint64_t plan_id);
+
+/* resident.cu: a register's plan slot for a flush, its sub-passes on the
+ * device (see there); split: as split.cu runs them. */
+struct p2_graph *p2_sub_plan(struct p2_dev *d,
+	const struct phase2_pass *passes, size_t npass,
+	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id,
+	bool split, bool *hit);
+
+/* split.cu: registers of middle width, a coset shared by four threads:
+ * whether a register's flush of this form runs there, and its launches, as
+ * p2_resident_run. */
+bool p2_split_ok(const struct p2_dev *d, int form);
+int p2_split_run(struct p2_dev *d, const struct phase2_pass *passes,
 	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
 	uint64_t plan_id);
 

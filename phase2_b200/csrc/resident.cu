@@ -24,98 +24,14 @@
 #define LOG_SUBSYS "engine"
 #include "log.h"
 
-/* all four pairs of a coset step by step: a warp is nearly alone on its
- * scheduler here, so independent FP64 operations have to come from it */
-#define P2_ROT_GROUP 4
-#define P2_LIFT_GROUP 4
-#include "p2_kernels.cuh"
-#include "sub_core.h"
+#include "p2_sub.cuh"
 
 #define P2_RES_MIN_QB 3
 #define P2_RES_MAX_QB 14
 #define P2_RES_TPB 256
 /* samples: many run at once, so a block may take a whole register */
 #define P2_RES_SMP_TPB 1024
-#define P2_RES_SLOTS (1 << P2_SUB_SPAN)
 #define P2_RES_SMEM (16 << 13) /* the most amplitudes of a block, 2^13 */
-
-/* ---- shared memory of the cluster --------------------------------------- */
-
-template <bool CL>
-__device__ __forceinline__ uint32_t p2_res_addr(uint32_t base, uint32_t pos,
-	uint32_t kc)
-{
-	uint32_t a = base + ((pos & ((1u << kc) - 1u)) << 4);
-	if constexpr (CL) {
-		const uint32_t rank = pos >> kc;
-		asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a)
-			: "r"(a), "r"(rank));
-	}
-	return a;
-}
-
-template <bool CL>
-__device__ __forceinline__ void p2_res_ld(uint32_t a, double &re, double &im)
-{
-	if constexpr (CL)
-		asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
-			: "=d"(re), "=d"(im) : "r"(a) : "memory");
-	else
-		asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
-			: "=d"(re), "=d"(im) : "r"(a) : "memory");
-}
-
-template <bool CL>
-__device__ __forceinline__ void p2_res_st(uint32_t a, double re, double im)
-{
-	if constexpr (CL)
-		asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};"
-			:: "r"(a), "d"(re), "d"(im) : "memory");
-	else
-		asm volatile("st.shared.v2.f64 [%0], {%1, %2};"
-			:: "r"(a), "d"(re), "d"(im) : "memory");
-}
-
-template <bool CL> __device__ __forceinline__ void p2_res_barrier()
-{
-	if constexpr (CL)
-		asm volatile("barrier.cluster.arrive.release.aligned;\n"
-			     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-	else
-		__syncthreads();
-}
-
-/* The rotation (key) on a coset of 8 slots: the exact FP64 update, or the
- * lifted one in FP64. */
-template <bool X, int K>
-__device__ __forceinline__ void p2_sub_rot(double (&re)[P2_RES_SLOTS],
-	double (&im)[P2_RES_SLOTS], double c, double s, uint32_t sm)
-{
-	if constexpr (X)
-		p2_rot_lift<P2_SUB_SPAN, (K >> 1), (K & 1)>(re, im, c, s, sm);
-	else
-		p2_rot<P2_SUB_SPAN, (K >> 1), (K & 1)>(re, im, c, s, sm, 0u);
-}
-
-#define P2_CASE_S(K)                                                           \
-	case K:                                                                \
-		p2_sub_rot<X, K>(re, im, q.c, q.s, sm);                        \
-		break;
-
-template <bool X>
-__device__ __forceinline__ void p2_sub_apply(const struct p2_sub_rec &q,
-	double (&re)[P2_RES_SLOTS], double (&im)[P2_RES_SLOTS], uint32_t sm)
-{
-	switch (q.key) {
-		P2_CASE_S(0) P2_CASE_S(1) P2_CASE_S(2) P2_CASE_S(3)
-		P2_CASE_S(4) P2_CASE_S(5) P2_CASE_S(6) P2_CASE_S(7)
-		P2_CASE_S(8) P2_CASE_S(9) P2_CASE_S(10) P2_CASE_S(11)
-		P2_CASE_S(12) P2_CASE_S(13) P2_CASE_S(14) P2_CASE_S(15)
-	default:
-		break;
-	}
-}
-#undef P2_CASE_S
 
 /* ---- the kernel ---------------------------------------------------------- */
 
@@ -375,12 +291,13 @@ static uint64_t hash_words(uint64_t h, const void *p, size_t n)
  * P2_GRAPH_SLOTS plans of the register by plan id (the same flush again) or
  * by content, or built and uploaded into the least recently used slot
  * (stream order keeps the copy behind the launches that read the slot).
+ * split: for split.cu, each pass's sub-passes on tiles of its own.
  * *hit: found.  NULL on failure.
  */
-static struct p2_graph *res_plan(struct p2_dev *d,
+struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	const struct phase2_pass *passes, size_t npass,
 	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id,
-	bool *hit)
+	bool split, bool *hit)
 {
 	struct p2_graph *lru = &d->graphs[0];
 	d->graph_clock++;
@@ -413,6 +330,8 @@ static struct p2_graph *res_plan(struct p2_dev *d,
 		/* keep the device buffer of a resident plan */
 		free(lru->passes);
 		free(lru->recs);
+		free(lru->split);
+		lru->split = NULL;
 		lru->nsub = 0;
 	} else {
 		p2_graph_drop(d, lru);
@@ -424,7 +343,10 @@ static struct p2_graph *res_plan(struct p2_dev *d,
 	lru->nrec = nrec;
 	lru->plan_id = 0;
 	lru->used = 0;
-	if (!lru->passes || !lru->recs)
+	if (split)
+		lru->split = (struct p2_split_pass *)malloc(
+			npass * sizeof *lru->split);
+	if (!lru->passes || !lru->recs || (split && !lru->split))
 		goto fail;
 	memcpy(lru->passes, passes, npass * sizeof *passes);
 	memcpy(lru->recs, recs, nrec * sizeof *recs);
@@ -439,9 +361,16 @@ static struct p2_graph *res_plan(struct p2_dev *d,
 		struct p2_sub *const ss = (struct p2_sub *)(sr + nrec);
 		uint32_t n = 0;
 		for (size_t i = 0; i < npass; i++)
-			n += p2_sub_split(&passes[i], recs + passes[i].rot_off,
-				d->nqb, passes[i].rot_off, ss + n,
-				sr + passes[i].rot_off);
+			if (split) {
+				p2_split_build(d->nqb, &passes[i], recs,
+					&lru->split[i], n, ss + n, sr);
+				n += lru->split[i].nsub;
+			} else {
+				n += p2_sub_split(&passes[i],
+					recs + passes[i].rot_off, d->nqb,
+					passes[i].rot_off, ss + n,
+					sr + passes[i].rot_off);
+			}
 		const size_t bytes = nrec * sizeof *sr + n * sizeof *ss;
 		if (bytes > lru->d_cap) {
 			p2_scratch_free(lru->d_recs, d->stream);
@@ -575,8 +504,8 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
 	uint64_t plan_id)
 {
 	bool hit;
-	struct p2_graph *g = res_plan(d, passes, npass, recs, nrec, plan_id,
-		&hit);
+	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
+		false, &hit);
 	if (!g)
 		return -1;
 	d->graph_replays += hit;

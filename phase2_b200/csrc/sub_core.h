@@ -206,4 +206,78 @@ P2_HD uint32_t p2_sub_split(const struct phase2_pass *ps,
 	return n;
 }
 
+/* ---- tiles of one pass (split.cu) --------------------------------------- */
+
+#define P2_SPLIT_BITS 10 /* amplitudes of a tile, log2 */
+
+/* A pass as k_pass_split takes it (span 3..5), and its sub-passes. */
+struct p2_split_pass {
+	struct phase2_pass pass;
+	uint32_t sub_off, nsub;
+};
+
+/*
+ * Sub-passes of pass `in` on tiles of 2^10 amplitudes: 2^(10 - span)
+ * consecutive representatives (the tile-local index's low bits) and their
+ * slots (its high bits).  The records' z are local, the pass's phase masks
+ * are kept in pad1 (a tile adds its representatives' part of the parity).
+ * recs, sr: the flush's records and their repacked copies.
+ */
+static inline void p2_split_build(uint32_t nqb, const struct phase2_pass *in,
+	const struct phase2_rot_rec *recs, struct p2_split_pass *out,
+	uint32_t sub_off, struct p2_sub *subs, struct p2_sub_rec *sr)
+{
+	struct phase2_pass *p = &out->pass;
+	*p = *in;
+	/* at least three dimensions: padding by unit vectors off the pivots,
+	 * which leave the pairs' order as it is */
+	for (uint32_t q = 0; p->span < P2_SUB_SPAN && q < nqb; q++) {
+		uint32_t at = 0;
+		while (at < p->span && p->piv[at] < q)
+			at++;
+		if (at < p->span && p->piv[at] == q)
+			continue;
+		for (uint32_t k = p->span; k > at; k--)
+			p->piv[k] = p->piv[k - 1];
+		p->piv[at] = (uint8_t)q;
+		p->basis[p->span++] = UINT64_C(1) << q;
+	}
+	const uint32_t M = p->span, LB = P2_SPLIT_BITS - M;
+	struct phase2_pass v;
+	memset(&v, 0, sizeof v);
+	v.span = M;
+	v.nrot = p->nrot;
+	v.rot_off = p->rot_off;
+	v.scale = p->scale;
+	for (uint32_t k = 0; k < M; k++) {
+		v.basis[k] = UINT64_C(1) << (LB + k);
+		v.piv[k] = (uint8_t)(LB + k);
+	}
+	uint64_t lane[P2_SPLIT_BITS];
+	for (uint32_t j = 0; j < LB; j++) {
+		lane[j] = UINT64_C(1) << j;
+		for (uint32_t k = 0; k < M; k++) {
+			const uint32_t q = p->piv[k];
+			lane[j] = ((lane[j] >> q) << (q + 1)) |
+				(lane[j] & ((UINT64_C(1) << q) - 1));
+		}
+	}
+	struct phase2_rot_rec r[P2_MAX_ROTS_PER_PASS];
+	for (uint32_t i = 0; i < p->nrot; i++) {
+		r[i] = recs[p->rot_off + i];
+		uint64_t z = 0;
+		for (uint32_t j = 0; j < LB; j++)
+			z |= (uint64_t)parity64(lane[j] & r[i].z) << j;
+		for (uint32_t k = 0; k < M; k++)
+			z |= (uint64_t)parity64(p->basis[k] & r[i].z)
+				<< (LB + k);
+		r[i].z = z;
+	}
+	out->sub_off = sub_off;
+	out->nsub = p2_sub_split(&v, r, P2_SPLIT_BITS, p->rot_off, subs,
+		sr + p->rot_off);
+	for (uint32_t i = 0; i < p->nrot; i++)
+		sr[p->rot_off + i].pad1 = recs[p->rot_off + i].z;
+}
+
 #endif /* P2_SUB_CORE_H */

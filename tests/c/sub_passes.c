@@ -2,7 +2,8 @@
  * Checks csrc/sub_core.h on the host: the sub-passes a plan is cut into
  * give the amplitudes of its passes bit for bit (the lifted update, whose
  * pairs are ordered), enumerate every amplitude once, cover every rotation
- * in order, and stay inside their staging limits.  Prints "ok" and returns
+ * in order, and stay inside their staging limits; and the same for the
+ * sub-passes on tiles of one pass (p2_split_build).  Prints "ok" and returns
  * 0, or names the first case that fails.
  */
 #include <math.h>
@@ -111,6 +112,71 @@ static const char *run_sub(double *a, uint32_t n, const struct p2_sub *h,
 	return NULL;
 }
 
+/* One pass through its tiles, as k_pass_split walks them. */
+static const char *run_split(double *a, uint32_t n,
+	const struct p2_split_pass *sp, const struct p2_sub *subs,
+	const struct p2_sub_rec *recs, char *seen)
+{
+	const struct phase2_pass *p = &sp->pass;
+	const uint32_t M = p->span, LB = P2_SPLIT_BITS - M, UL = 7 - LB;
+	uint32_t piv[PHASE2_MAX_SPAN], at[1 << P2_SPLIT_BITS];
+	if (M < 3 || M > 5)
+		return "split span";
+	for (uint32_t k = 0; k < M; k++)
+		piv[k] = p->piv[k];
+	memset(seen, 0, (size_t)1 << n);
+	for (uint32_t b = 0; b < (1u << n) >> P2_SPLIT_BITS; b++) {
+		const uint32_t xb = insert_zeros(b << LB, piv, (int)M);
+		for (uint32_t t = 0; t < 128; t++)
+			for (uint32_t i = 0; i < 8; i++) {
+				uint32_t g = insert_zeros((b << LB) +
+						(t & ((1u << LB) - 1)),
+					piv, (int)M);
+				for (uint32_t k = 0; k < UL; k++)
+					if (t >> (LB + k) & 1)
+						g ^= (uint32_t)p->basis[k];
+				for (uint32_t k = 0; k < 3; k++)
+					if (i >> k & 1)
+						g ^= (uint32_t)p->basis[UL + k];
+				if (g >> n || seen[g]++)
+					return "split enumeration";
+				at[t + 128 * i] = g;
+			}
+		for (uint32_t i = 0; i < sp->nsub; i++) {
+			const struct p2_sub *h = &subs[sp->sub_off + i];
+			for (uint32_t t = 0; t < 128; t++) {
+				uint32_t y = insert_zeros(t, h->piv, P2_SUB_SPAN);
+				uint32_t idx[8];
+				const uint32_t y0 = y;
+				for (int k = 0; k < P2_SUB_SPAN; k++)
+					if (parity64(y0 & h->orient[k]))
+						y ^= h->slot[k];
+				for (uint32_t u = 0; u < 8; u++) {
+					uint32_t g = y;
+					for (int k = 0; k < P2_SUB_SPAN; k++)
+						if (u >> k & 1)
+							g ^= h->slot[k];
+					if (g >> P2_SPLIT_BITS)
+						return "split slot";
+					idx[u] = at[g];
+				}
+				for (uint32_t r = 0; r < h->nrot; r++) {
+					const struct p2_sub_rec *q =
+						&recs[h->rot_off + r];
+					const int s = parity64(y & q->z) ^
+						parity64(xb & q->pad1);
+					rotate(a, idx, P2_SUB_SPAN, q->key >> 1,
+						q->key & 1, q->c, q->s,
+						q->sm ^ (0u - (uint32_t)s));
+				}
+			}
+		}
+	}
+	for (size_t i = 0; i < (size_t)2 << n; i++)
+		a[i] = (float)(p->scale < 0 ? -a[i] : a[i]);
+	return NULL;
+}
+
 int main(void)
 {
 	enum { R = 400, N = 1 << 14 };
@@ -119,7 +185,7 @@ int main(void)
 	static struct phase2_rot_rec rc[R];
 	static struct p2_sub ss[R];
 	static struct p2_sub_rec sr[R];
-	static double a[2 * N], b[2 * N];
+	static double a[2 * N], b[2 * N], c[2 * N];
 	static char seen[N];
 	srand48(1);
 	for (int trial = 0; trial < 300; trial++) {
@@ -145,7 +211,7 @@ int main(void)
 			lrand48() % 4 ? 0 : 1 + (int)(lrand48() % 9),
 			P2_DEFAULT_PAD_SPAN, form, 0, 0, ps, rc);
 		for (size_t i = 0; i < (size_t)2 << n; i++)
-			a[i] = b[i] = (float)(drand48() - 0.5);
+			a[i] = b[i] = c[i] = (float)(drand48() - 0.5);
 		uint32_t ns = 0, covered = 0;
 		for (long p = 0; p < np; p++) {
 			run_pass(a, n, &ps[p], rc + ps[p].rot_off);
@@ -164,6 +230,16 @@ int main(void)
 			bad = "coverage";
 		if (!bad && memcmp(a, b, (size_t)16 << n))
 			bad = "bits";
+		ns = 0;
+		for (long p = 0; p < np && !bad && n >= P2_SPLIT_BITS; p++) {
+			struct p2_split_pass sp;
+			p2_split_build(n, &ps[p], rc, &sp, ns, ss + ns, sr);
+			ns += sp.nsub;
+			bad = run_split(c, n, &sp, ss, sr, seen);
+		}
+		if (!bad && n >= P2_SPLIT_BITS &&
+			memcmp(a, c, (size_t)16 << n))
+			bad = "split bits";
 		if (bad) {
 			printf("trial %d, %u qubits: %s\n", trial, n, bad);
 			return 1;

@@ -1,6 +1,7 @@
-"""Small registers held on chip (one launch a flush): the oracle's bits at
-the widths where the block count changes, long sub-passes, and more plans
-than the register keeps; FP32 states against the persistent kernel's bits."""
+"""Registers whose passes run as sub-passes (held on chip up to 14 qubits, a
+tile a block up to 19): the oracle's bits at the widths where the kernel or
+the block count changes, every span, long sub-passes, and more plans than
+the register keeps."""
 
 import numpy as np
 import pytest
@@ -21,7 +22,7 @@ def _rots(n, k, seed):
     return t.flip, t.phase, rng.uniform(-4, 4, k)
 
 
-@pytest.mark.parametrize("n", [3, 4, 8, 11, 12, 13, 14, 15])
+@pytest.mark.parametrize("n", [3, 4, 8, 11, 12, 13, 14, 15, 17, 19, 20])
 def test_bits_and_plans(n, oracle_lib):
     rng = np.random.Generator(np.random.PCG64(n))
     amp = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
@@ -36,7 +37,7 @@ def test_bits_and_plans(n, oracle_lib):
         assert np.array_equal(r.get_state(), amp)
 
 
-@pytest.mark.parametrize("n", [5, 11, 13, 14])
+@pytest.mark.parametrize("n", [5, 11, 13, 14, 15, 19])
 def test_forms_share_a_register(n, oracle_lib):
     """Flushes of the FP32-arithmetic form (pass kernels, replayed from
     graphs) and of the mixed form (on chip) take turns on one register's
@@ -59,3 +60,17 @@ def test_forms_share_a_register(n, oracle_lib):
             assert np.max(np.abs(r.get_state() - amp)) < 1e-5
     finally:
         p2.set_fp32_form(old)
+
+
+@pytest.mark.parametrize("fusion", [(1, 1), (2, 0), (4, 3)])
+@pytest.mark.parametrize("n", [10, 14, 16, 19])
+def test_spans(n, fusion, oracle_lib):
+    flip, phase, phi = _rots(n, 80, 7 * n)
+    amp = np.zeros(1 << n, dtype=np.complex128)
+    amp[5] = 1.0
+    with Register(n, p2.PREC_FP64) as r:
+        r.set_fusion(*fusion)
+        r.set_state(amp)
+        r.paulirot(flip, phase, phi)
+        assert np.array_equal(r.get_state(),
+                              oracle_lib.rotate(amp, n, flip, phase, phi))
