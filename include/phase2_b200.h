@@ -328,12 +328,15 @@ struct phase2_stats {
 	double pass_ms;     /* device time of timed pass launches (CUDA events) */
 	uint64_t h2d_bytes; /* host-to-device bytes copied for this register */
 	uint64_t d2h_bytes; /* device-to-host bytes copied for this register */
-	uint64_t graph_replays; /* flushes launched from a captured CUDA graph
-				 * (a plan seen before, e.g. every Trotter
-				 * step after the second; registers of up to
-				 * 24 qubits) */
-	uint64_t sweeps;    /* state round trips: one per pass kernel, one per
-			     * sweep kernel (several passes, phase2_set_sweep) */
+	uint64_t graph_replays; /* flushes launched from a plan kept on the
+				 * device (seen before, e.g. every Trotter
+				 * step after the first or second): a captured
+				 * CUDA graph (registers of up to 24 qubits),
+				 * or kept sub-passes and tile runs */
+	uint64_t sweeps;    /* state round trips as planned: one per pass, one
+			     * per sweep kernel (phase2_set_sweep) or tile run
+			     * (FP64, 20 qubits up: several passes' rotations);
+			     * a register held on chip counts its passes */
 	uint64_t timed_sweeps; /* round trips inside pass_ms */
 };
 

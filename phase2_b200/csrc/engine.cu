@@ -962,6 +962,7 @@ void p2_graph_drop(struct p2_dev *d, struct p2_graph *g)
 	free(g->passes);
 	free(g->recs);
 	free(g->split);
+	free(g->tiles);
 	memset(g, 0, sizeof *g);
 }
 
@@ -998,6 +999,11 @@ int p2_status_check(struct p2_dev *d)
 		return -1;
 	}
 	return 0;
+}
+
+extern "C" void p2d_set_tiles(struct p2_dev *d, int on)
+{
+	d->tiles = on;
 }
 
 extern "C" int p2d_zero(struct p2_dev *d)
@@ -1511,8 +1517,10 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 {
 	if (npass == 0)
 		return 0;
-	const bool split = p2_split_ok(d, passes[0].form);
-	const bool resident = split || p2_resident_ok(d, passes[0].form);
+	const int form = passes[0].form;
+	const bool split = p2_split_ok(d, form);
+	const bool tile = p2_tile_ok(d, form, npass, nrec);
+	const bool resident = split || tile || p2_resident_ok(d, form);
 	struct p2_graph *g = resident
 		? NULL
 		: graph_for(d, passes, npass, recs, nrec);
@@ -1530,7 +1538,14 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	if (d->timing && !resident)
 		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	long launches;
-	if (resident) {
+	if (tile) {
+		size_t trips;
+		if (p2_tile_run(d, passes, npass, recs, nrec, plan_id,
+			    &trips) < 0)
+			return -1;
+		d->launches += trips;
+		launches = (long)trips;
+	} else if (resident) {
 		/* counted as one state round trip a pass, as planned */
 		if ((split ? p2_split_run : p2_resident_run)(d, passes, npass,
 			    recs, nrec, plan_id) < 0)

@@ -43,6 +43,8 @@ struct p2_graph {
 	size_t d_cap;
 	uint32_t nsub;
 	struct p2_split_pass *split; /* per pass (split.cu), or NULL */
+	struct p2_tile *tiles;       /* ntile runs (tile.cu), or NULL */
+	uint32_t ntile;
 	uint64_t plan_id; /* the caller's number of this plan (0: none) */
 	int status;     /* the graph holds kernels that write d_status */
 	uint64_t used;
@@ -56,6 +58,7 @@ struct p2_dev {
 	void *state;
 	cudaStream_t stream;
 	int sm_count;
+	int tiles;        /* passes may be regrouped (p2d_set_tiles) */
 	int device;       /* of the shell (engine.cu) */
 	uint64_t context;
 
@@ -209,11 +212,12 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
 	uint64_t plan_id);
 
 /* resident.cu: a register's plan slot for a flush, its sub-passes on the
- * device (see there); split: as split.cu runs them. */
+ * device (see there). */
+enum p2_plan_kind { P2_PLAN_RESIDENT, P2_PLAN_SPLIT, P2_PLAN_TILE };
 struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	const struct phase2_pass *passes, size_t npass,
 	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id,
-	bool split, bool *hit);
+	enum p2_plan_kind kind, bool *hit);
 
 /* split.cu: registers of middle width, a coset shared by four threads:
  * whether a register's flush of this form runs there, and its launches, as
@@ -247,6 +251,14 @@ struct p2_res_samples {
 bool p2_resident_samples_ok(const struct p2_dev *d, int form);
 cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
 	uint32_t g);
+
+/* tile.cu: FP64 registers beyond the caches: whether a flush's rotations run
+ * regrouped into tile runs, and their launches, as p2_resident_run; *trips:
+ * state round trips. */
+bool p2_tile_ok(const struct p2_dev *d, int form, size_t npass, size_t nrec);
+int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
+	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
+	uint64_t plan_id, size_t *trips);
 
 /* lift_bulk.cu: one FP32 pass of the FP64-arithmetic form on a kernel
  * whose next cosets are staged in shared memory, by bulk copies (variant

@@ -63,6 +63,11 @@ void p2d_destroy(struct p2_dev *d);
  * staging, freed pool memory of the current device). */
 void p2d_release(void);
 
+/* on: the flush's rotations may be grouped otherwise than in its passes
+ * where that gives the same bits (FP64; full fusion only: a caller that
+ * limits spans or rotations a pass asks for those passes). */
+void p2d_set_tiles(struct p2_dev *d, int on);
+
 int p2d_zero(struct p2_dev *d);
 int p2d_set(struct p2_dev *d, const uint64_t *idx, const double *z, size_t n);
 int p2d_get(struct p2_dev *d, const uint64_t *idx, double *z, size_t n);

@@ -96,6 +96,7 @@ int qreg_init_prec(struct qreg *reg, uint32_t nqb, int prec)
 		free(b);
 		return -1;
 	}
+	p2d_set_tiles(b->dev, b->max_span == PHASE2_MAX_SPAN && b->max_rots == 0);
 	reg->qb_lo = nqb;
 	reg->qb_hi = 0;
 	reg->namp = UINT64_C(1) << nqb;
@@ -272,6 +273,7 @@ int qreg_set_fusion(struct qreg *reg, int max_span, int max_rots)
 		return -1;
 	b->max_span = max_span;
 	b->max_rots = max_rots;
+	p2d_set_tiles(b->dev, max_span == PHASE2_MAX_SPAN && max_rots == 0);
 	return 0;
 }
 

@@ -25,6 +25,7 @@
 #include "log.h"
 
 #include "p2_sub.cuh"
+#include "tile_core.h"
 
 #define P2_RES_MIN_QB 3
 #define P2_RES_MAX_QB 14
@@ -291,13 +292,14 @@ static uint64_t hash_words(uint64_t h, const void *p, size_t n)
  * P2_GRAPH_SLOTS plans of the register by plan id (the same flush again) or
  * by content, or built and uploaded into the least recently used slot
  * (stream order keeps the copy behind the launches that read the slot).
- * split: for split.cu, each pass's sub-passes on tiles of its own.
+ * kind: sub-passes of the register (here), of each pass on tiles of its own
+ * (split.cu), or tile runs (tile.cu).
  * *hit: found.  NULL on failure.
  */
 struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	const struct phase2_pass *passes, size_t npass,
 	const struct phase2_rot_rec *recs, size_t nrec, uint64_t plan_id,
-	bool split, bool *hit)
+	enum p2_plan_kind kind, bool *hit)
 {
 	struct p2_graph *lru = &d->graphs[0];
 	d->graph_clock++;
@@ -331,8 +333,10 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
 		free(lru->passes);
 		free(lru->recs);
 		free(lru->split);
+		free(lru->tiles);
 		lru->split = NULL;
-		lru->nsub = 0;
+		lru->tiles = NULL;
+		lru->nsub = lru->ntile = 0;
 	} else {
 		p2_graph_drop(d, lru);
 	}
@@ -343,10 +347,15 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	lru->nrec = nrec;
 	lru->plan_id = 0;
 	lru->used = 0;
-	if (split)
+	if (kind == P2_PLAN_SPLIT)
 		lru->split = (struct p2_split_pass *)malloc(
 			npass * sizeof *lru->split);
-	if (!lru->passes || !lru->recs || (split && !lru->split))
+	if (kind == P2_PLAN_TILE)
+		lru->tiles = (struct p2_tile *)malloc(
+			nrec * sizeof *lru->tiles);
+	if (!lru->passes || !lru->recs ||
+		(kind == P2_PLAN_SPLIT && !lru->split) ||
+		(kind == P2_PLAN_TILE && !lru->tiles))
 		goto fail;
 	memcpy(lru->passes, passes, npass * sizeof *passes);
 	memcpy(lru->recs, recs, nrec * sizeof *recs);
@@ -360,8 +369,19 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
 		struct p2_sub_rec *const sr = (struct p2_sub_rec *)stage;
 		struct p2_sub *const ss = (struct p2_sub *)(sr + nrec);
 		uint32_t n = 0;
-		for (size_t i = 0; i < npass; i++)
-			if (split) {
+		size_t sub_bytes = sizeof *ss;
+		if (kind == P2_PLAN_TILE) {
+			lru->ntile = p2_tile_build(passes, npass, recs, nrec,
+				lru->tiles, (struct p2_tile_sub *)ss,
+				(struct p2_tile_rec *)sr, &n);
+			sub_bytes = sizeof(struct p2_tile_sub);
+			struct p2_tile *fit = (struct p2_tile *)realloc(
+				lru->tiles, lru->ntile * sizeof *fit);
+			if (fit)
+				lru->tiles = fit;
+		}
+		for (size_t i = 0; i < npass && kind != P2_PLAN_TILE; i++)
+			if (kind == P2_PLAN_SPLIT) {
 				p2_split_build(d->nqb, &passes[i], recs,
 					&lru->split[i], n, ss + n, sr);
 				n += lru->split[i].nsub;
@@ -371,7 +391,7 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
 					passes[i].rot_off, ss + n,
 					sr + passes[i].rot_off);
 			}
-		const size_t bytes = nrec * sizeof *sr + n * sizeof *ss;
+		const size_t bytes = nrec * sizeof *sr + n * sub_bytes;
 		if (bytes > lru->d_cap) {
 			p2_scratch_free(lru->d_recs, d->stream);
 			lru->d_recs = NULL;
@@ -505,7 +525,7 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
 {
 	bool hit;
 	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
-		false, &hit);
+		P2_PLAN_RESIDENT, &hit);
 	if (!g)
 		return -1;
 	d->graph_replays += hit;

@@ -198,7 +198,7 @@ int p2_split_run(struct p2_dev *d, const struct phase2_pass *passes,
 {
 	bool hit;
 	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
-		true, &hit);
+		P2_PLAN_SPLIT, &hit);
 	if (!g)
 		return -1;
 	d->graph_replays += hit;

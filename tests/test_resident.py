@@ -1,16 +1,19 @@
-"""Small registers held on chip: the cut of passes into sub-passes, on the
-CPU, against the passes themselves (tests/c/sub_passes.c)."""
+"""Passes cut into sub-passes and tile runs, on the CPU, against the passes
+and the rotations themselves (tests/c/sub_passes.c, tests/c/tile_runs.c)."""
 
 import subprocess
+
+import pytest
 
 from conftest import ROOT
 
 
-def test_sub_passes_equal_passes(tmp_path):
-    exe = tmp_path / "sub_passes"
+@pytest.mark.parametrize("name", ["sub_passes", "tile_runs"])
+def test_cut_equals_passes(name, tmp_path):
+    exe = tmp_path / name
     subprocess.run(["gcc", "-O2", "-std=gnu11", "-ffp-contract=off",
                     f"-I{ROOT}/include", f"-I{ROOT}/phase2_b200/csrc",
-                    str(ROOT / "tests/c/sub_passes.c"), "-o", str(exe),
+                    str(ROOT / f"tests/c/{name}.c"), "-o", str(exe),
                     "-lm"], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
