@@ -466,6 +466,44 @@ __global__ void k_scatter(ST *__restrict__ st, const uint64_t *__restrict__ idx,
 			p2_st(st, idx[i], val[2 * i], val[2 * i + 1]);
 }
 
+/* A few amplitudes passed with the launch (an overlap's determinants, a
+ * trial state): no index or value buffers, no copies, and for the scatter no
+ * synchronisation; the gather writes to pinned host memory.  A 12-qubit
+ * Trotter step's overlap took a 64 KiB download, a preparation two uploads
+ * and two synchronisations. */
+#define P2_FEW 32
+struct p2_few {
+	uint64_t idx[P2_FEW];
+	double val[2 * P2_FEW];
+	uint32_t n;
+};
+
+template <typename ST>
+__global__ void k_scatter_few(ST *__restrict__ st,
+	const __grid_constant__ struct p2_few f)
+{
+	const uint32_t i = threadIdx.x;
+	if (i >= f.n)
+		return;
+	for (uint32_t j = i + 1; j < f.n; ++j)
+		if (f.idx[j] == f.idx[i])
+			return; /* a later write of the same amplitude holds */
+	p2_st(st, f.idx[i], f.val[2 * i], f.val[2 * i + 1]);
+}
+
+template <typename ST>
+__global__ void k_gather_few(const ST *__restrict__ st,
+	const __grid_constant__ struct p2_few f, double *__restrict__ out)
+{
+	const uint32_t i = threadIdx.x;
+	if (i < f.n) {
+		double re, im;
+		p2_ld(st, f.idx[i], re, im);
+		out[2 * i] = re;
+		out[2 * i + 1] = im;
+	}
+}
+
 /* Neumaier: s + c carries the running sum and its rounding error. */
 __device__ __forceinline__ void p2_neumaier(double &s, double &c, double v)
 {
@@ -1030,7 +1068,26 @@ extern "C" int p2d_set(struct p2_dev *d, const uint64_t *idx, const double *z,
 {
 	if (n == 0)
 		return 0;
-	if (check_idx(d, idx, n) < 0 || io_reserve(d, n) < 0)
+	if (check_idx(d, idx, n) < 0)
+		return -1;
+	if (n <= P2_FEW) {
+		struct p2_few f;
+		memset(&f, 0, sizeof f);
+		f.n = (uint32_t)n;
+		memcpy(f.idx, idx, n * sizeof *idx);
+		memcpy(f.val, z, n * 2 * sizeof *z);
+		if (d->prec == PHASE2_PREC_FP64)
+			k_scatter_few<<<1, P2_FEW, 0, d->stream>>>(
+				(double2 *)d->state, f);
+		else
+			k_scatter_few<<<1, P2_FEW, 0, d->stream>>>(
+				(float2 *)d->state, f);
+		d->launches++;
+		d->h2d_bytes += n * (sizeof(uint64_t) + 2 * sizeof(double));
+		CUDA_OK(cudaGetLastError(), "scatter launch");
+		return 0;
+	}
+	if (io_reserve(d, n) < 0)
 		return -1;
 	CUDA_OK(cudaStreamSynchronize(d->stream), "sync before set");
 	memcpy(d->h_idx, idx, n * sizeof *idx);
@@ -1061,6 +1118,25 @@ extern "C" int p2d_get(struct p2_dev *d, const uint64_t *idx, double *z,
 		return 0;
 	if (check_idx(d, idx, n) < 0 || io_reserve(d, n) < 0)
 		return -1;
+	if (n <= P2_FEW) {
+		struct p2_few f;
+		memset(&f, 0, sizeof f);
+		f.n = (uint32_t)n;
+		memcpy(f.idx, idx, n * sizeof *idx);
+		if (d->prec == PHASE2_PREC_FP64)
+			k_gather_few<<<1, P2_FEW, 0, d->stream>>>(
+				(const double2 *)d->state, f, d->h_val);
+		else
+			k_gather_few<<<1, P2_FEW, 0, d->stream>>>(
+				(const float2 *)d->state, f, d->h_val);
+		d->launches++;
+		d->h2d_bytes += n * sizeof(uint64_t);
+		d->d2h_bytes += n * 2 * sizeof(double);
+		CUDA_OK(cudaGetLastError(), "gather launch");
+		CUDA_OK(cudaStreamSynchronize(d->stream), "gather");
+		memcpy(z, d->h_val, n * 2 * sizeof(double));
+		return p2_status_check(d);
+	}
 	CUDA_OK(cudaStreamSynchronize(d->stream), "sync before get");
 	memcpy(d->h_idx, idx, n * sizeof *idx);
 	CUDA_OK(cudaMemcpyAsync(d->d_idx, d->h_idx, n * sizeof *idx,
@@ -1596,18 +1672,17 @@ static int part_reserve(struct p2_dev *d, unsigned blocks)
 /* Run k_reduce_final over `blocks` partials and download the result. */
 static int reduce_finish(struct p2_dev *d, unsigned blocks, double out[2])
 {
+	/* the result goes straight to pinned host memory */
+	if (io_reserve(d, 1) < 0)
+		return -1;
 	k_reduce_final<<<1, P2_RED_TPB, 0, d->stream>>>(d->d_part, blocks,
-		d->d_part + 2 * (size_t)blocks);
+		d->h_val);
 	d->launches += 1;
 	CUDA_OK(cudaGetLastError(), "reduce launch");
-	double h[2];
-	CUDA_OK(cudaMemcpyAsync(h, d->d_part + 2 * (size_t)blocks, sizeof h,
-			cudaMemcpyDeviceToHost, d->stream),
-		"download reduction");
 	CUDA_OK(cudaStreamSynchronize(d->stream), "reduce");
-	d->d2h_bytes += sizeof h;
-	out[0] = h[0];
-	out[1] = h[1];
+	d->d2h_bytes += 2 * sizeof(double);
+	out[0] = d->h_val[0];
+	out[1] = d->h_val[1];
 	return p2_status_check(d);
 }
 
@@ -1625,6 +1700,9 @@ static int reduce(struct p2_dev *d, const double2 *trial, double out[2])
 	d->launches += 1;
 	return reduce_finish(d, blocks, out);
 }
+
+/* Tables up to this size go up in one copy. */
+#define P2_CM_STAGE ((size_t)512 << 10)
 
 /* Upload the expansion tables (occupations, weights, determinants) into
  * the register's table buffer; *p receives the five device pointers. */
@@ -1649,13 +1727,24 @@ static int cm_upload(struct p2_dev *d, const uint64_t *occ_a, size_t Ma,
 		CUDA_OK(cudaMalloc((void **)&d->d_cm, total), "alloc tables");
 		d->cm_cap = total;
 	}
-	for (int k = 0; k < 5; k++) {
+	for (int k = 0; k < 5; k++)
 		p[k] = d->d_cm + off[k];
+	if (total <= P2_CM_STAGE) {
+		/* one copy through the pinned staging */
+		unsigned char *h = (unsigned char *)p2_stage_reserve(d,
+			(total + 31) / 32);
+		if (!h)
+			return -1;
+		for (int k = 0; k < 5; k++)
+			if (sz[k])
+				memcpy(h + off[k], src[k], sz[k]);
+		return p2_stage_upload(d, d->d_cm, total);
+	}
+	for (int k = 0; k < 5; k++)
 		if (sz[k])
 			CUDA_OK(cudaMemcpyAsync(p[k], src[k], sz[k],
 					cudaMemcpyHostToDevice, d->stream),
 				"upload tables");
-	}
 	d->h2d_bytes += sz[0] + sz[1] + sz[2] + sz[3] + sz[4];
 	return 0;
 }

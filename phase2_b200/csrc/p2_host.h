@@ -33,8 +33,8 @@ void p2_settings_from_env(void);
  * rotations (q) and amplitude writes (w*).  At most one of them is
  * non-empty: queuing into one drains the other first.  Reads drain both.
  * Registers of up to P2_HOST_COPY_QB qubits keep a host copy of the state
- * (host_copy) after a read, valid until the next change, so that long runs
- * of single-amplitude reads cost one download.
+ * (host_copy) after a second read, valid until the next change, so that long
+ * runs of single-amplitude reads cost one download.
  */
 #define P2_HOST_COPY_QB 16
 
@@ -52,7 +52,7 @@ struct p2_qreg {
 	double *wval;
 	size_t wlen, wcap;
 	double *host_copy;
-	int host_copy_valid;
+	enum { COPY_STALE = 0, COPY_VALID, COPY_READ_ONCE } host_copy_valid;
 	struct p2_prog *rec; /* recording instead of executing, or NULL */
 	/* input of the plan held in passes/recs (a flush whose queue is
 	 * byte-identical, with the same settings, reuses it: every Trotter

@@ -62,6 +62,9 @@ static void zero_free(void *p, size_t bytes)
 		munmap(p, bytes);
 }
 
+/* Amplitudes read one by one gather on the device up to this many. */
+#define QREG_FEW 32
+
 static struct p2_qreg *B(const struct qreg *reg)
 {
 	return (struct p2_qreg *)reg->backend;
@@ -295,7 +298,7 @@ void qreg_paulirot(struct qreg *reg, struct paulis code_hi,
 		return;
 	if (drain_writes(b) < 0)
 		return;
-	b->host_copy_valid = 0;
+	b->host_copy_valid = COPY_STALE;
 	/* Operators beyond the register's qubits are dropped, as the
 	 * reference's hi/lo split does (phase2/paulis.c:165-180). */
 	const uint64_t m = reg->qb_lo >= 64 ? ~UINT64_C(0)
@@ -355,7 +358,7 @@ int qreg_setamps(struct qreg *reg, const uint64_t *idx,
 	memcpy(b->widx + b->wlen, idx, sizeof *idx * n);
 	memcpy(b->wval + 2 * b->wlen, z, sizeof(double) * 2 * n);
 	b->wlen += n;
-	b->host_copy_valid = 0;
+	b->host_copy_valid = COPY_STALE;
 	return 0;
 }
 
@@ -374,13 +377,16 @@ int qreg_getamps(struct qreg *reg, const uint64_t *idx, _Complex double *z,
 	if (qreg_flush(reg) < 0)
 		return -1;
 	double *out = (double *)z; /* _Complex double = (re, im) */
-	if (b->host_copy) {
-		if (!b->host_copy_valid) {
+	/* the first read after a change gathers its few amplitudes; a second
+	 * one brings the whole state */
+	const int gather = n <= QREG_FEW && b->host_copy_valid == COPY_STALE;
+	if (b->host_copy && !gather) {
+		if (b->host_copy_valid != COPY_VALID) {
 			if (p2d_get_state(b->dev, b->host_copy) < 0) {
 				b->error = -1;
 				return -1;
 			}
-			b->host_copy_valid = 1;
+			b->host_copy_valid = COPY_VALID;
 		}
 		for (size_t i = 0; i < n; i++) {
 			out[2 * i] = b->host_copy[2 * idx[i]];
@@ -392,6 +398,8 @@ int qreg_getamps(struct qreg *reg, const uint64_t *idx, _Complex double *z,
 		b->error = -1;
 		return -1;
 	}
+	if (gather)
+		b->host_copy_valid = COPY_READ_ONCE;
 	return 0;
 }
 
@@ -422,15 +430,9 @@ void qreg_zero(struct qreg *reg)
 			b->error = -1;
 		return;
 	}
-	if (p2d_zero(b->dev) < 0) {
+	b->host_copy_valid = COPY_STALE;
+	if (p2d_zero(b->dev) < 0)
 		b->error = -1;
-		b->host_copy_valid = 0;
-		return;
-	}
-	if (b->host_copy) {
-		memset(b->host_copy, 0, sizeof(double) * 2 * reg->namp);
-		b->host_copy_valid = 1;
-	}
 }
 
 int qreg_get_state(struct qreg *reg, double *out)
@@ -438,7 +440,7 @@ int qreg_get_state(struct qreg *reg, double *out)
 	struct p2_qreg *b = B(reg);
 	if (!b || recording(b, "qreg_get_state") || qreg_flush(reg) < 0)
 		return -1;
-	if (b->host_copy && b->host_copy_valid) {
+	if (b->host_copy && b->host_copy_valid == COPY_VALID) {
 		memcpy(out, b->host_copy, sizeof(double) * 2 * reg->namp);
 		return 0;
 	}
@@ -452,7 +454,7 @@ int qreg_set_state(struct qreg *reg, const double *in)
 		return -1;
 	b->qlen = 0;
 	b->wlen = 0;
-	b->host_copy_valid = 0;
+	b->host_copy_valid = COPY_STALE;
 	return p2d_set_state(b->dev, in);
 }
 
@@ -506,7 +508,7 @@ static int slab_copy(struct qreg *reg, uint32_t bit, uint32_t val,
 		qreg_flush(reg) < 0)
 		return -1;
 	if (put)
-		b->host_copy_valid = 0;
+		b->host_copy_valid = COPY_STALE;
 	return p2d_slab_copy(b->dev, bit, val, first, count, buf, put);
 }
 
@@ -530,8 +532,8 @@ int qreg_slab_swap(struct qreg *a, struct qreg *b, uint32_t bit,
 		recording(bb, "qreg_slab_swap") || qreg_flush(a) < 0 ||
 		qreg_flush(b) < 0)
 		return -1;
-	ba->host_copy_valid = 0;
-	bb->host_copy_valid = 0;
+	ba->host_copy_valid = COPY_STALE;
+	bb->host_copy_valid = COPY_STALE;
 	return p2d_slab_swap(ba->dev, bb->dev, bit, val_a, val_b);
 }
 
@@ -541,7 +543,7 @@ int p2_qreg_record(struct qreg *reg, struct p2_prog *pg)
 	if (!b || b->rec || qreg_flush(reg) < 0)
 		return -1;
 	b->rec = pg;
-	b->host_copy_valid = 0;
+	b->host_copy_valid = COPY_STALE;
 	return 0;
 }
 
@@ -586,7 +588,7 @@ struct p2_dev *p2_qreg_direct(struct qreg *reg)
 	if (!b || recording(b, "coefficient-matrix state") ||
 		qreg_flush(reg) < 0)
 		return NULL;
-	b->host_copy_valid = 0;
+	b->host_copy_valid = COPY_STALE;
 	return b->dev;
 }
 
