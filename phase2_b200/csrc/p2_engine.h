@@ -252,6 +252,32 @@ bool p2_resident_samples_ok(const struct p2_dev *d, int form);
 cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
 	uint32_t g);
 
+/*
+ * resident.cu: a batch whose registers all fit on chip.  A program's ops: a
+ * run of sub-passes subs[a .. a + b) (records recs), or P2_OP_ZERO / WRITE /
+ * GATHER with a, b as in struct p2_op.  Whether a register of this form can
+ * be in such a batch, and the launch of g programs on d's stream (nqb: the
+ * widest register; even: as many programs of the largest one's work as the
+ * batch's work makes; ctl[i].end_ns and the complement of the start time in
+ * *start as k_batch leaves them).
+ */
+#define P2_RES_RUN 0x100
+struct p2_res_op {
+	uint32_t kind, a, b;
+};
+struct p2_res_prog {
+	void *state;
+	const struct p2_res_op *ops;
+	const struct p2_sub *subs;
+	const struct p2_sub_rec *recs;
+	uint32_t nqb, nops;
+};
+bool p2_resident_prog_ok(const struct p2_dev *d, int form);
+cudaError_t p2_resident_progs(const struct p2_dev *d, uint32_t nqb, uint32_t g,
+	uint32_t even, const struct p2_res_prog *progs, const uint64_t *widx,
+	const double *wval, const uint64_t *gidx, double2 *gout,
+	struct p2_bctl *ctl, unsigned long long *start);
+
 /* tile.cu: FP64 registers beyond the caches: whether a flush's rotations run
  * regrouped into tile runs, and their launches, as p2_resident_run; *trips:
  * state round trips. */

@@ -774,4 +774,11 @@ struct p2_bctl {
 	unsigned long long line[13];
 };
 
+__device__ __forceinline__ unsigned long long p2_globaltimer()
+{
+	unsigned long long t;
+	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+	return t;
+}
+
 #endif /* P2_KERNELS_CUH */

@@ -28,6 +28,7 @@
 #include "tile_core.h"
 
 #define P2_RES_MIN_QB 3
+#define P2_RES_MIN_SHARE 5 /* log2 of a block's least share of a register */
 #define P2_RES_MAX_QB 14
 #define P2_RES_TPB 256
 /* samples: many run at once, so a block may take a whole register */
@@ -243,6 +244,91 @@ __global__ void __launch_bounds__(P2_RES_SMP_TPB) k_resident_smp(
 					(p2_sub_swz(first + i) & low), re, im);
 			p2_st((ST *)a.state, first + i, re, im);
 		}
+}
+
+/*
+ * A batch's programs (batch.cu), one cluster of 2^lb blocks each: the
+ * register's state stays on chip from the first op to the last.  A register
+ * too narrow to share out lies in the first block alone; the others keep the
+ * barriers.
+ */
+template <typename ST, bool X, bool CL>
+__global__ void __launch_bounds__(P2_RES_SMP_TPB) k_resident_prog(
+	const struct p2_res_prog *__restrict__ progs, uint32_t lb,
+	const uint64_t *__restrict__ widx, const double *__restrict__ wval,
+	const uint64_t *__restrict__ gidx, double2 *__restrict__ gout,
+	struct p2_bctl *__restrict__ ctl, unsigned long long *start)
+{
+	extern __shared__ __align__(16) unsigned char p2_res_dyn[];
+	__shared__ __align__(16) struct p2_res_stagebuf sb;
+	const uint32_t tid = threadIdx.x, nt = blockDim.x;
+	const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(p2_res_dyn);
+	const uint32_t rank = CL ? blockIdx.x & ((1u << lb) - 1u) : 0u;
+	const uint32_t who = blockIdx.x >> lb;
+	const struct p2_res_prog a = progs[who];
+	const bool shared_out = CL && a.nqb >= lb + P2_RES_MIN_SHARE;
+	const uint32_t kc = shared_out ? a.nqb - lb : a.nqb;
+	const uint32_t low = (1u << kc) - 1u, first = rank << kc;
+	const bool mine = shared_out || rank == 0;
+	const uint32_t n = mine ? 1u << kc : 0u;
+	/* threads of a block beyond its share of the register idle */
+	const uint32_t share = 1u << (kc - P2_SUB_SPAN);
+	const uint32_t t = mine && tid < share ? rank * share + tid : ~0u;
+	if (blockIdx.x == 0 && tid == 0)
+		atomicMax(start, ~p2_globaltimer());
+	for (uint32_t i = tid; i < n; i += nt) {
+		double re, im;
+		p2_ld((const ST *)a.state, first + i, re, im);
+		p2_res_st<false>(sbase + 16 * (p2_sub_swz(first + i) & low), re,
+			im);
+	}
+	for (uint32_t o = 0; o < a.nops; ++o) {
+		const struct p2_res_op op = a.ops[o];
+		if (op.kind == P2_RES_RUN) {
+			p2_res_run<X, CL>(a.nqb, kc, sbase, t, a.subs + op.a,
+				op.b, a.recs, sb);
+			continue;
+		}
+		/* between two runs a block touches only its own amplitudes */
+		__syncthreads();
+		if (op.kind == P2_OP_ZERO) {
+			for (uint32_t i = tid; i < n; i += nt)
+				p2_res_st<false>(sbase + 16 * i, 0.0, 0.0);
+		} else if (op.kind == P2_OP_WRITE) {
+			/* in order: later writes win */
+			for (uint32_t e = op.a; tid == 0 && e < op.a + op.b; ++e) {
+				const uint32_t g = (uint32_t)widx[e];
+				if (!mine || g >> kc != rank)
+					continue;
+				double re = wval[2 * e], im = wval[2 * e + 1];
+				if (sizeof(ST) == 8) {
+					re = (double)__double2float_rn(re);
+					im = (double)__double2float_rn(im);
+				}
+				p2_res_st<false>(sbase + 16 *
+						(p2_sub_swz(g) & low), re, im);
+			}
+		} else {
+			for (uint32_t e = op.a + tid; e < op.a + op.b; e += nt) {
+				const uint32_t g = (uint32_t)gidx[e];
+				if (!mine || g >> kc != rank)
+					continue;
+				double re, im;
+				p2_res_ld<false>(sbase + 16 *
+						(p2_sub_swz(g) & low), re, im);
+				gout[e] = make_double2(re, im);
+			}
+		}
+		__syncthreads();
+	}
+	for (uint32_t i = tid; i < n; i += nt) {
+		double re, im;
+		p2_res_ld<false>(sbase + 16 * (p2_sub_swz(first + i) & low), re,
+			im);
+		p2_st((ST *)a.state, first + i, re, im);
+	}
+	if (rank == 0 && tid == 0)
+		ctl[who].end_ns = p2_globaltimer();
 }
 
 /* ---- host side ----------------------------------------------------------- */
@@ -546,11 +632,11 @@ int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
  * samples 1581 / 1512 / 1485 / 1577 / 1724, 128 samples 1812 / 2424 / 3651 /
  * 3964 / 4559).  A block holds 2^13 amplitudes at most.
  */
-static uint32_t res_sample_blocks(const struct p2_dev *d, uint64_t g)
+static uint32_t res_sample_blocks(uint32_t nqb, int sm_count, uint64_t g)
 {
-	const uint32_t least = d->nqb > 13 ? d->nqb - 13 : 0;
-	uint32_t lb = res_log_blocks(d->nqb);
-	while (lb > least && (g << lb) > (uint64_t)d->sm_count / 2)
+	const uint32_t least = nqb > 13 ? nqb - 13 : 0;
+	uint32_t lb = res_log_blocks(nqb);
+	while (lb > least && (g << lb) > (uint64_t)sm_count / 2)
 		lb--;
 	return lb;
 }
@@ -583,9 +669,50 @@ cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
 	uint32_t g)
 {
 	a.nqb = d->nqb;
-	a.lb = res_sample_blocks(d, g);
+	a.lb = res_sample_blocks(d->nqb, d->sm_count, g);
 	a.state = d->state;
 	return d->prec == PHASE2_PREC_FP64
 		? res_launch_samples<double2, false>(d, a, g)
 		: res_launch_samples<float2, true>(d, a, g);
+}
+
+/* ---- batch programs ------------------------------------------------------- */
+
+bool p2_resident_prog_ok(const struct p2_dev *d, int form)
+{
+	if (!res_width_ok(d, form))
+		return false;
+	/* any width's clusters: the batch's widest register chooses them */
+	return d->prec == PHASE2_PREC_FP64
+		? res_clusters<k_resident_prog<double2, false, true>>(true) >= 16 &&
+			res_clusters<k_resident_prog<double2, false, false>>(
+				false) >= 1
+		: res_clusters<k_resident_prog<float2, true, true>>(true) >= 16 &&
+			res_clusters<k_resident_prog<float2, true, false>>(
+				false) >= 1;
+}
+
+template <typename ST, bool X>
+static cudaError_t res_launch_progs(uint32_t nqb, uint32_t lb, uint32_t g,
+	cudaStream_t stream, const struct p2_res_prog *progs,
+	const uint64_t *widx, const double *wval, const uint64_t *gidx,
+	double2 *gout, struct p2_bctl *ctl, unsigned long long *start)
+{
+	return res_launch(lb ? k_resident_prog<ST, X, true>
+			     : k_resident_prog<ST, X, false>,
+		g << lb, nqb, lb, stream, progs, lb, widx, wval, gidx, gout, ctl,
+		start);
+}
+
+cudaError_t p2_resident_progs(const struct p2_dev *d, uint32_t nqb, uint32_t g,
+	uint32_t even, const struct p2_res_prog *progs, const uint64_t *widx,
+	const double *wval, const uint64_t *gidx, double2 *gout,
+	struct p2_bctl *ctl, unsigned long long *start)
+{
+	const uint32_t lb = res_sample_blocks(nqb, d->sm_count, even);
+	return d->prec == PHASE2_PREC_FP64
+		? res_launch_progs<double2, false>(nqb, lb, g, d->stream, progs,
+			  widx, wval, gidx, gout, ctl, start)
+		: res_launch_progs<float2, true>(nqb, lb, g, d->stream, progs,
+			  widx, wval, gidx, gout, ctl, start);
 }
