@@ -180,7 +180,8 @@ int phase2_set_sweep_kernel(int on);
  * Modes: OFF (host loop), ON (device whenever the register qualifies),
  * AUTO (default: device for qualifying registers of at most
  * PHASE2_DEVICE_SAMPLING_AUTO_QB qubits, where samples run concurrently;
- * wider registers keep the host loop, whose passes already fill the GPU).
+ * wider registers, and one or two samples of 15 qubits or more, keep the
+ * host loop).
  * Step writers: under AUTO a driver with a step writer attached keeps the
  * host loop, which calls the writer as each sample completes (a writer
  * that flushes per step stays crash-consistent and can report progress);

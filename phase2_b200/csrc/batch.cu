@@ -36,7 +36,7 @@ __device__ __forceinline__ void p2_batch_pass_tile(float2 *st,
 	for (uint32_t j = 0; j < cpt; ++j) {
 		const uint64_t t = t0 + (uint64_t)j * 32;
 		if (t < nrep)
-			p2_lift32_coset<M, uint32_t, true>(st,
+			p2_lift32_coset<M, uint32_t, true, false>(st,
 				p2_rep_t<M, uint32_t>((uint32_t)t, p), pb, srec,
 				p.nrot, negm);
 	}

@@ -212,6 +212,16 @@ static int persistent_reg_ok(const struct qreg *reg)
 	return b && p2d_batch_ok(b->dev);
 }
 
+/* One or two samples of a register that does not fit on chip: the persistent
+ * kernel's op costs 10 us whether or not other samples share the launch, a
+ * pass of the host loop 3.4-13 us (500 draws, ms a call, host loop / device:
+ * 17 qubits, 1, 2, 4 samples 0.51 / 1.10, 0.97 / 1.12, 1.86 / 1.16; 20
+ * qubits 0.80 / 1.49, 1.57 / 1.99, 3.01 / 3.15). */
+static int few_samples(const struct circ *ct)
+{
+	return ct->reg.qb_lo >= 15 && ct->vals.len <= 2;
+}
+
 /* Registers that device sampling (p2d_sampled_device) takes under the
  * current mode: those the persistent kernel runs (FP64, or FP32 in either
  * form; at most 31 qubits) with a multi-determinant trial state; AUTO
@@ -227,7 +237,8 @@ static int device_sampling_ok(const struct circ *ct,
 	const struct p2_qreg *b = ct->reg.backend;
 	if (p2_cfg.device_sampling == PHASE2_DEVICE_SAMPLING_OFF ||
 		(p2_cfg.device_sampling == PHASE2_DEVICE_SAMPLING_AUTO &&
-			(ct->reg.qb_lo > PHASE2_DEVICE_SAMPLING_AUTO_QB || sw)))
+			(ct->reg.qb_lo > PHASE2_DEVICE_SAMPLING_AUTO_QB || sw ||
+				few_samples(ct))))
 		return 0;
 	return b && b->rec == NULL && persistent_reg_ok(&ct->reg) &&
 		ct->stprep_kind == STPREP_MULTIDET && ct->md.len > 0;

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(P2_TPB, M >= 5 ? 3 : p2_min_blocks(M))
  * registers back.  Half the registers of k_pass_lift (20 resident warps
  * per SM at M = 5) and no conversions.
  */
-template <int M, typename IT>
+template <int M, typename IT, bool PK>
 __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 	k_pass_lift32(float2 *__restrict__ st, uint64_t nrep,
 		struct phase2_pass p,
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 		t < nrep; t += stride)
-		p2_lift32_coset<M, IT, false>(st, p2_rep_t<M, IT>((IT)t, p),
+		p2_lift32_coset<M, IT, false, PK>(st, p2_rep_t<M, IT>((IT)t, p),
 			pb, srec, nrot, negm);
 }
 
@@ -345,7 +345,7 @@ __device__ __forceinline__ void p2_heavy_run(double2 *hv, IT x,
  * the run with FP32 FMAs, the same bits as k_pass_lift32.  The warps walk
  * the cosets 32 at a time, so every lane is present for the heavy runs.
  */
-template <int M, typename IT>
+template <int M, typename IT, bool PK>
 __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 	k_pass_lift32h(float2 *__restrict__ st, uint64_t nrep,
 		struct phase2_pass p,
@@ -419,9 +419,8 @@ __global__ void __launch_bounds__(P2_TPB, p2_lift32_blocks(M))
 		if (active && !heavy) {
 			for (uint32_t r = 0; r < nrot; ++r) {
 				const struct p2_lift32_rec q = srec[r];
-				const uint32_t sm =
-					q.sm ^ (0u - p2_parity(x & (IT)q.z));
-				p2_apply_lift32<M>(q, re, im, sm);
+				p2_apply_lift32<M, PK>(q, re, im,
+					p2_parity(x & (IT)q.z));
 			}
 		}
 		if (active) {
@@ -1322,6 +1321,17 @@ static int launch_pass_t(struct p2_dev *d, const struct phase2_pass &p,
 	return 0;
 }
 
+template <int M, bool PK>
+static void (*lift32_kernel(bool narrow, bool mixed))(float2 *, uint64_t,
+	struct phase2_pass, const struct phase2_rot_rec *)
+{
+	if (mixed)
+		return narrow ? k_pass_lift32h<M, uint32_t, PK>
+			      : k_pass_lift32h<M, uint64_t, PK>;
+	return narrow ? k_pass_lift32<M, uint32_t, PK>
+		      : k_pass_lift32<M, uint64_t, PK>;
+}
+
 /* One FP32 pass in the lifted form of the pass: FP32 arithmetic
  * (k_pass_lift32) or FP64 arithmetic (k_pass_lift); 32-bit index
  * arithmetic up to 31 qubits. */
@@ -1335,24 +1345,21 @@ static int launch_lift_t(struct p2_dev *d, const struct phase2_pass &p,
 	const unsigned grid = grid_for(d, nrep, P2_TPB, per_sm);
 	float2 *const sv = (float2 *)d->state;
 	const bool narrow = d->nqb <= 31;
-	if (p.form == PHASE2_FORM_LIFTED_F32) {
-		if (narrow)
-			CUDA_OK(p2_launch(k_pass_lift32<M, uint32_t>, grid, P2_TPB, 0,
-				d->stream, sv, nrep, p, recs),
-			"pass launch");
-		else
-			CUDA_OK(p2_launch(k_pass_lift32<M, uint64_t>, grid, P2_TPB, 0,
-				d->stream, sv, nrep, p, recs),
-			"pass launch");
-	} else if (p.form == PHASE2_FORM_LIFTED_MIXED &&
-		d->nqb >= P2_MIXED_MIN_QB) {
-		if (narrow)
-			CUDA_OK(p2_launch(k_pass_lift32h<M, uint32_t>, grid, P2_TPB, 0,
-				d->stream, sv, nrep, p, recs),
-			"pass launch");
-		else
-			CUDA_OK(p2_launch(k_pass_lift32h<M, uint64_t>, grid, P2_TPB, 0,
-				d->stream, sv, nrep, p, recs),
+	if (p.form == PHASE2_FORM_LIFTED_F32 ||
+		(p.form == PHASE2_FORM_LIFTED_MIXED &&
+			d->nqb >= P2_MIXED_MIN_QB)) {
+		/* long passes are bound by issue slots, where packed sign steps
+		 * save one of eight a pair, short ones by memory, where they
+		 * cost (28 qubits, mixed form, 1e12 rotations x amplitudes a
+		 * second, packed / not: 37 rotations a pass 5.41 / 4.99, 18
+		 * 4.42 / 4.13, 5.4 2.03 / 2.12) */
+		const bool mixed = p.form == PHASE2_FORM_LIFTED_MIXED;
+		void (*const fn)(float2 *, uint64_t, struct phase2_pass,
+			const struct phase2_rot_rec *) = p.nrot > 10
+			? lift32_kernel<M, true>(narrow, mixed)
+			: lift32_kernel<M, false>(narrow, mixed);
+		CUDA_OK(p2_launch(fn, grid, P2_TPB, 0, d->stream, sv, nrep, p,
+				recs),
 			"pass launch");
 	} else if (p.form == PHASE2_FORM_LIFTED ||
 		p.form == PHASE2_FORM_LIFTED_MIXED) {

@@ -496,17 +496,51 @@ __device__ __forceinline__ float p2_fsgn(float v, uint32_t mask)
  * phi) / s in FP64 (plan.c); the angle of the three shears is fixed by the
  * product t s (their trace is 2 (1 - t s)), so rounding t to FP32 leaves a
  * relative angle error of at most 2^-25.  The signs go onto the
- * coefficients (one XOR each on a 32-bit register).
+ * coefficients: the pairs are walked in Gray code order, and a step
+ * multiplies t and s by the +-1 with which the sign changes along its slot
+ * bit (exact).  A pair is then seven or eight instructions of the FMA pipe;
+ * extracting each pair's sign bit took five of the ALU, which has half the
+ * rate and was the busiest pipe on long passes (ncu, 38 rotations a pass:
+ * ALU 60 %, FMA 35 %, issue 74 %).
  */
-template <int M, int U, int ODD>
+/* Pair number of step i of the walk over a rotation's pairs, and the bit in
+ * which it differs from the one before (i > 0). */
+__host__ __device__ constexpr int p2_gray(int i)
+{
+	return i ^ (i >> 1);
+}
+
+__host__ __device__ constexpr int p2_gray_bit(int i)
+{
+	return i & 1 ? 0 : i & 2 ? 1 : i & 4 ? 2 : i & 8 ? 3 : 4;
+}
+
+/* t and s times the +-1 f of a step: as one packed product (PK) or two. */
+template <bool PK>
+__device__ __forceinline__ void p2_lift32_step(float &t, float &s, float f)
+{
+	if constexpr (PK) {
+		const float2 v = __fmul2_rn(make_float2(t, s), make_float2(f, f));
+		t = v.x;
+		s = v.y;
+	} else {
+		t *= f;
+		s *= f;
+	}
+}
+
+template <int M, int U, int ODD, bool PK>
 __device__ __forceinline__ void p2_rot_lift32(float (&re)[1 << M],
-	float (&im)[1 << M], float t, float s, uint32_t sm)
+	float (&im)[1 << M], const float t, const float s,
+	const float (&m)[PHASE2_MAX_SPAN])
 {
 	if constexpr (U == 0) {
+		float st = t, ss = s;
 #pragma unroll
-		for (int u = 0; u < (1 << M); ++u) {
-			const uint32_t g = p2_bitmask(sm, u);
-			const float st = p2_fsgn(t, g), ss = p2_fsgn(s, g);
+		for (int i = 0; i < (1 << M); ++i) {
+			const int u = p2_gray(i);
+			if (i > 0)
+				p2_lift32_step<PK>(st, ss, m[p2_gray_bit(i)]);
 			if constexpr (ODD) {
 				re[u] = fmaf(-st, im[u], re[u]);
 				im[u] = fmaf(ss, re[u], im[u]);
@@ -525,31 +559,39 @@ __device__ __forceinline__ void p2_rot_lift32(float (&re)[1 << M],
 		constexpr int H = p2_hibit(U);
 		constexpr int NP = 1 << (M - 1);
 		constexpr int G = NP < P2_LIFT32_GROUP ? NP : P2_LIFT32_GROUP;
+		float t0 = t, s0 = s;
 #pragma unroll
 		for (int g0 = 0; g0 < NP; g0 += G) {
 			float st[G], ss[G];
 #pragma unroll
 			for (int j = 0; j < G; ++j) {
-				const uint32_t b = p2_bitmask(sm, p2_ins0(g0 + j, H));
-				st[j] = p2_fsgn(t, b);
-				ss[j] = p2_fsgn(s, b);
+				if (g0 + j > 0) {
+					const int b = p2_gray_bit(g0 + j);
+					p2_lift32_step<PK>(t0, s0,
+						m[b < H ? b : b + 1]);
+				}
+				st[j] = t0;
+				ss[j] = s0;
 			}
 			if constexpr (ODD) {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g0 + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g0 + j), H),
+						  w = u ^ U;
 					re[u] = fmaf(-st[j], im[w], re[u]);
 					im[u] = fmaf(st[j], re[w], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g0 + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g0 + j), H),
+						  w = u ^ U;
 					re[w] = fmaf(-ss[j], im[u], re[w]);
 					im[w] = fmaf(ss[j], re[u], im[w]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g0 + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g0 + j), H),
+						  w = u ^ U;
 					re[u] = fmaf(-st[j], im[w], re[u]);
 					im[u] = fmaf(st[j], re[w], im[u]);
 				}
@@ -560,7 +602,8 @@ __device__ __forceinline__ void p2_rot_lift32(float (&re)[1 << M],
 				float2 yu[G], yw[G];
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g0 + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g0 + j), H),
+						  w = u ^ U;
 					yu[j] = make_float2(re[u], im[u]);
 					yw[j] = make_float2(re[w], im[w]);
 				}
@@ -578,7 +621,8 @@ __device__ __forceinline__ void p2_rot_lift32(float (&re)[1 << M],
 						yw[j], yu[j]);
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g0 + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g0 + j), H),
+						  w = u ^ U;
 					re[u] = yu[j].x;
 					im[u] = yu[j].y;
 					re[w] = yw[j].x;
@@ -590,24 +634,28 @@ __device__ __forceinline__ void p2_rot_lift32(float (&re)[1 << M],
 }
 
 /* A lifted record as the FP32 kernel reads it. */
-struct p2_lift32_rec {
-	float t, s;
+struct __align__(16) p2_lift32_rec {
 	uint64_t z;
-	uint32_t sm;  /* smask */
 	uint32_t key; /* U << 1 | odd */
+	uint32_t sm;  /* smask */
+	float t, s;
+	float m[PHASE2_MAX_SPAN]; /* +-1: the sign's change with slot bit k */
+	float pad;
 };
 
 #define P2_CASE_L32(K)                                                         \
 	case K:                                                                \
 		if constexpr ((K) < (2 << M))                                  \
-			p2_rot_lift32<M, ((K) >> 1), ((K)&1)>(re, im, q.t,     \
-				q.s, sm);                                      \
+			p2_rot_lift32<M, ((K) >> 1), ((K)&1), PK>(re, im, t,   \
+				s, q.m);                                       \
 		break;
 
-template <int M>
+template <int M, bool PK>
 __device__ __forceinline__ void p2_apply_lift32(const struct p2_lift32_rec &q,
-	float (&re)[1 << M], float (&im)[1 << M], uint32_t sm)
+	float (&re)[1 << M], float (&im)[1 << M], uint32_t parity)
 {
+	const uint32_t b = (q.sm ^ parity) << 31; /* slot 0's sign */
+	const float t = p2_fsgn(q.t, b), s = p2_fsgn(q.s, b);
 	switch (q.key) {
 		P2_CASE_L32(0) P2_CASE_L32(1) P2_CASE_L32(2) P2_CASE_L32(3)
 		P2_CASE_L32(4) P2_CASE_L32(5) P2_CASE_L32(6) P2_CASE_L32(7)
@@ -647,6 +695,10 @@ __device__ __forceinline__ struct p2_lift32_rec p2_lift32_of(
 	o.s = (float)in.s; /* an FP32 value: exact */
 	o.z = in.z;
 	o.sm = in.smask;
+#pragma unroll
+	for (int k = 0; k < PHASE2_MAX_SPAN; ++k)
+		o.m[k] = in.W >> k & 1 ? -1.f : 1.f;
+	o.pad = 0.f;
 	o.key = ((uint32_t)in.U << 1) | in.odd;
 	return o;
 }
@@ -658,7 +710,7 @@ __device__ __forceinline__ struct p2_lift32_rec p2_lift32_of(
  * persistent batch kernel, whose blocks read what other blocks of the same
  * launch wrote).
  */
-template <int M, typename IT, bool CG>
+template <int M, typename IT, bool CG, bool PK>
 __device__ __forceinline__ void p2_lift32_coset(float2 *__restrict__ st, IT x,
 	const IT (&pb)[M > 0 ? M : 1], const struct p2_lift32_rec *srec,
 	uint32_t nrot, uint32_t negm)
@@ -677,8 +729,7 @@ __device__ __forceinline__ void p2_lift32_coset(float2 *__restrict__ st, IT x,
 	}
 	for (uint32_t r = 0; r < nrot; ++r) {
 		const struct p2_lift32_rec q = srec[r];
-		const uint32_t sm = q.sm ^ (0u - p2_parity(x & (IT)q.z));
-		p2_apply_lift32<M>(q, re, im, sm);
+		p2_apply_lift32<M, PK>(q, re, im, p2_parity(x & (IT)q.z));
 	}
 	const IT xs = p2_opaque(x);
 #pragma unroll

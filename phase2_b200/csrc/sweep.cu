@@ -120,8 +120,8 @@ __device__ __forceinline__ void p2_sweep_pass(float2 *__restrict__ st,
 		}
 		for (uint32_t r = 0; r < nrot; ++r) {
 			const struct p2_lift32_rec q = srec[P.rec_off + r];
-			const uint32_t sm = q.sm ^ (0u - p2_parity(x & (uint32_t)q.z));
-			p2_apply_lift32<M>(q, re, im, sm);
+			p2_apply_lift32<M, false>(q, re, im,
+				p2_parity(x & (uint32_t)q.z));
 		}
 		const uint32_t xs = (uint32_t)p2_opaque(x);
 		const uint32_t sxs = (uint32_t)p2_opaque(sx);
