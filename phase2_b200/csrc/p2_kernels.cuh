@@ -289,10 +289,13 @@ __device__ __forceinline__ void p2_prefetch(double2 *stage, const double2 *st,
  *   y_u += t q_u y_w;  y_w += s q_w y_u;  y_u += t q_u y_w,
  * q_u = sigma (odd ? i : 1), q_w = -conj(q_u), t = tan(phi/2): every update
  * writes the register it reads, so a case needs no temporaries and leaves
- * no moves behind.  The sign goes onto the two coefficients (one XOR on the
- * high word of each, sigma t and sigma s); the FMAs then take them with
- * free operand negations.  Rounding is symmetric under negation, so this
- * gives the same bits as flipping the partner's sign around the shears.
+ * no moves behind.  The sign goes onto the two coefficients (sigma t and
+ * sigma s; the FMAs take them with free operand negations): the pairs are
+ * walked in Gray code order, and a step XORs the high word of each with the
+ * sign's change along its slot bit (extracting and placing every pair's bit
+ * anew cost 4-17 % of the rotation, most where few warps share a
+ * scheduler).  Rounding is symmetric under negation, so this gives the same
+ * bits as flipping the partner's sign around the shears.
  * U = 0 (the string is diagonal on the coset, and then odd = 1) is the
  * phase c + i sigma s, applied to (re, im) by the same three shears.
  *
@@ -308,10 +311,28 @@ __device__ __forceinline__ void p2_prefetch(double2 *stage, const double2 *st,
 #define P2_LIFT32_GROUP 4
 #endif
 
+/* Pair number of step i of the walk over a rotation's pairs, and the bit in
+ * which it differs from the one before (i > 0). */
+__host__ __device__ constexpr int p2_gray(int i)
+{
+	return i ^ (i >> 1);
+}
+
+__host__ __device__ constexpr int p2_gray_bit(int i)
+{
+	return i & 1 ? 0 : i & 2 ? 1 : i & 4 ? 2 : i & 8 ? 3 : 4;
+}
+
 template <int M, int U, int ODD>
 __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 	double (&im)[1 << M], double t, double s, uint32_t sm)
 {
+	/* the sign's change along slot bit k */
+	uint32_t mk[M > 0 ? M : 1];
+#pragma unroll
+	for (int k = 0; k < M; ++k)
+		mk[k] = ((sm << (31 - (1 << k))) ^ (sm << 31)) & 0x80000000u;
+	double t0 = p2_sgn(t, sm << 31), s0 = p2_sgn(s, sm << 31);
 	if constexpr (U == 0) {
 		constexpr int S = 1 << M;
 		constexpr int G = S < P2_LIFT_GROUP ? S : P2_LIFT_GROUP;
@@ -320,28 +341,39 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 			double st[G], ss[G];
 #pragma unroll
 			for (int j = 0; j < G; ++j) {
-				const uint32_t b = p2_bitmask(sm, g + j);
-				st[j] = p2_sgn(t, b);
-				ss[j] = p2_sgn(s, b);
+				if (g + j > 0) {
+					const uint32_t f = mk[p2_gray_bit(g + j)];
+					t0 = p2_sgn(t0, f);
+					s0 = p2_sgn(s0, f);
+				}
+				st[j] = t0;
+				ss[j] = s0;
 			}
 			if constexpr (ODD) {
 #pragma unroll
-				for (int j = 0; j < G; ++j)
-					re[g + j] = fma(-st[j], im[g + j], re[g + j]);
+				for (int j = 0; j < G; ++j) {
+					const int u = p2_gray(g + j);
+					re[u] = fma(-st[j], im[u], re[u]);
+				}
 #pragma unroll
-				for (int j = 0; j < G; ++j)
-					im[g + j] = fma(ss[j], re[g + j], im[g + j]);
+				for (int j = 0; j < G; ++j) {
+					const int u = p2_gray(g + j);
+					im[u] = fma(ss[j], re[u], im[u]);
+				}
 #pragma unroll
-				for (int j = 0; j < G; ++j)
-					re[g + j] = fma(-st[j], im[g + j], re[g + j]);
+				for (int j = 0; j < G; ++j) {
+					const int u = p2_gray(g + j);
+					re[u] = fma(-st[j], im[u], re[u]);
+				}
 			} else {
 				/* (c +- s) y with c = 1 - t s; a Hermitian string
 				 * that is diagonal on the coset never has it */
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
+					const int u = p2_gray(g + j);
 					const double k = ss[j] + fma(-t, s, 1.0);
-					re[g + j] *= k;
-					im[g + j] *= k;
+					re[u] *= k;
+					im[u] *= k;
 				}
 			}
 		}
@@ -354,45 +386,56 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 			double st[G], ss[G];
 #pragma unroll
 			for (int j = 0; j < G; ++j) {
-				const uint32_t b = p2_bitmask(sm, p2_ins0(g + j, H));
-				st[j] = p2_sgn(t, b);
-				ss[j] = p2_sgn(s, b);
+				if (g + j > 0) {
+					const int b = p2_gray_bit(g + j);
+					const uint32_t f = mk[b < H ? b : b + 1];
+					t0 = p2_sgn(t0, f);
+					s0 = p2_sgn(s0, f);
+				}
+				st[j] = t0;
+				ss[j] = s0;
 			}
 			if constexpr (ODD) {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[u] = fma(-st[j], im[w], re[u]);
 					im[u] = fma(st[j], re[w], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[w] = fma(-ss[j], im[u], re[w]);
 					im[w] = fma(ss[j], re[u], im[w]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[u] = fma(-st[j], im[w], re[u]);
 					im[u] = fma(st[j], re[w], im[u]);
 				}
 			} else {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[u] = fma(st[j], re[w], re[u]);
 					im[u] = fma(st[j], im[w], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[w] = fma(-ss[j], re[u], re[w]);
 					im[w] = fma(-ss[j], im[u], im[w]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(g + j, H), w = u ^ U;
+					const int u = p2_ins0(p2_gray(g + j), H),
+						  w = u ^ U;
 					re[u] = fma(st[j], re[w], re[u]);
 					im[u] = fma(st[j], im[w], im[u]);
 				}
@@ -503,18 +546,6 @@ __device__ __forceinline__ float p2_fsgn(float v, uint32_t mask)
  * rate and was the busiest pipe on long passes (ncu, 38 rotations a pass:
  * ALU 60 %, FMA 35 %, issue 74 %).
  */
-/* Pair number of step i of the walk over a rotation's pairs, and the bit in
- * which it differs from the one before (i > 0). */
-__host__ __device__ constexpr int p2_gray(int i)
-{
-	return i ^ (i >> 1);
-}
-
-__host__ __device__ constexpr int p2_gray_bit(int i)
-{
-	return i & 1 ? 0 : i & 2 ? 1 : i & 4 ? 2 : i & 8 ? 3 : 4;
-}
-
 /* t and s times the +-1 f of a step: as one packed product (PK) or two. */
 template <bool PK>
 __device__ __forceinline__ void p2_lift32_step(float &t, float &s, float f)

@@ -38,7 +38,7 @@
  * (programmatic dependent launch).
  */
 template <typename ST, bool X, int M>
-__global__ void __launch_bounds__(P2_SPLIT_TPB, 8) k_pass_split(
+__global__ void __launch_bounds__(P2_SPLIT_TPB, 7) k_pass_split(
 	ST *__restrict__ st, const struct phase2_pass p,
 	const struct p2_sub *__restrict__ subs, uint32_t nsub,
 	const struct p2_sub_rec *__restrict__ recs)
