@@ -645,15 +645,17 @@ bool p2_resident_samples_ok(const struct p2_dev *d, int form)
 {
 	if (!res_width_ok(d, form))
 		return false;
-	const uint32_t lb = res_log_blocks(d->nqb);
-	const unsigned most = d->prec == PHASE2_PREC_FP64
-		? (lb ? res_clusters<k_resident_smp<double2, false, true>>(true)
-		      : res_clusters<k_resident_smp<double2, false, false>>(
-				false))
-		: (lb ? res_clusters<k_resident_smp<float2, true, true>>(true)
-		      : res_clusters<k_resident_smp<float2, true, false>>(
-				false));
-	return most >= (1u << lb);
+	/* both kernels: the number of samples chooses between them */
+	const unsigned need = 1u << res_log_blocks(d->nqb);
+	return d->prec == PHASE2_PREC_FP64
+		? res_clusters<k_resident_smp<double2, false, true>>(true) >=
+				need &&
+			res_clusters<k_resident_smp<double2, false, false>>(
+				false) >= 1
+		: res_clusters<k_resident_smp<float2, true, true>>(true) >=
+				need &&
+			res_clusters<k_resident_smp<float2, true, false>>(
+				false) >= 1;
 }
 
 template <typename ST, bool X>

@@ -2,10 +2,14 @@
 count, several chunks of the host queue, head terms, repeated and unordered
 determinants; overlaps, final register and generator as on the host loop."""
 
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import phase2_b200 as p2
+from conftest import ROOT
 from phase2_b200 import Dets, workloads
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +50,19 @@ def test_cmpsit(n, length, depth, prec):
     t = workloads.jw_terms(n, 60, seed=n)
     d = workloads.hamming_dets(n, 2, n // 2, seed=n)
     _both("cmpsit", prec, n, t, d, 3, 2, length, depth, 0.05, 0.01, 99)
+
+
+@pytest.mark.parametrize("prec", ["FP64", "FP32"])
+@pytest.mark.parametrize("n,samples", [(12, 80), (13, 80), (14, 2)])
+def test_first_run_of_a_process(n, samples, prec):
+    """A process whose first register is wide: the kernel its sample count
+    chooses is configured without any other having run."""
+    code = (f"import phase2_b200 as p2\n"
+            f"from phase2_b200 import workloads as w\n"
+            f"p2.world_ensure(); p2.set_precision(p2.PREC_{prec})\n"
+            f"t = w.jw_terms({n}, 50, seed=1)\n"
+            f"d = w.hamming_dets({n}, 1, {n} // 2, seed=2)\n"
+            f"p2.set_device_sampling(True)\n"
+            f"assert len(p2.qdrift({n}, t, d, {samples}, 20, 0.05, 3))"
+            f" == {samples}\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
