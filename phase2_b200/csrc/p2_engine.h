@@ -252,6 +252,24 @@ bool p2_resident_samples_ok(const struct p2_dev *d, int form);
 cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
 	uint32_t g);
 
+/* onchip.cu: the same for many samples, a block each, by
+ * whole passes: sample s's passes of chunk c are passes[s * T + c *
+ * P2_QUEUE_FLUSH ..], npc[s * C + c] of them, their rot_off into recs. */
+struct p2_oc_samples {
+	uint32_t nqb, ndet, C;
+	uint64_t T, keep;
+	const struct phase2_pass *passes;
+	const uint32_t *npc;
+	const struct phase2_rot_rec *recs;
+	const uint64_t *widx;
+	const double *wval;
+	double2 *gout;
+	void *state;
+};
+bool p2_onchip_samples_ok(const struct p2_dev *d, int form, uint64_t samples);
+cudaError_t p2_onchip_samples(struct p2_dev *d, struct p2_oc_samples a,
+	uint32_t g);
+
 /*
  * resident.cu: a batch whose registers all fit on chip.  A program's ops: a
  * run of sub-passes subs[a .. a + b) (records recs), or P2_OP_ZERO / WRITE /

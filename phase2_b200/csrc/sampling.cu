@@ -472,7 +472,10 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		R = 1;
 	const uint32_t C = (uint32_t)((T + P2_QUEUE_FLUSH - 1) / P2_QUEUE_FLUSH);
 	/* registers that fit on chip: no state copies, no persistent kernel */
-	const bool res = T > 0 && p2_resident_samples_ok(d, job->form);
+	const bool whole = T > 0 && p2_onchip_samples_ok(d, job->form, samples);
+	const bool subs = T > 0 && !whole &&
+		p2_resident_samples_ok(d, job->form);
+	const bool res = whole || subs;
 	if (res) {
 		R = 1;
 		/* twice the scratch a rotation */
@@ -507,9 +510,9 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		sz[PROG] = (G * T + 3 * G) * sizeof(struct p2_op);
 		sz[NPC] = sz[POFF] = (G * C != 0 ? G * C : 1) * sizeof(uint32_t);
 		sz[SOFF] = G * sizeof(uint32_t);
-		sz[SUBT] = sz[SUB] = res ? GT * sizeof(struct p2_sub) : 0;
-		sz[SREC] = res ? GT * sizeof(struct p2_sub_rec) : 0;
-		sz[NSUB] = res ? sz[NPC] : 0;
+		sz[SUBT] = sz[SUB] = subs ? GT * sizeof(struct p2_sub) : 0;
+		sz[SREC] = subs ? GT * sizeof(struct p2_sub_rec) : 0;
+		sz[NSUB] = subs ? sz[NPC] : 0;
 		if (res)
 			sz[PROG] = sz[GIDX] = 0;
 		sz[REGS] = R * (sizeof(struct p2_binst) +
@@ -664,7 +667,7 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 				(struct phase2_pass *)(b + off[PASS]),
 				(struct phase2_rot_rec *)(b + off[REC]), npc,
 				(struct p2_sub *)(b + off[SUBT]),
-				res ? (struct p2_sub *)(b + off[SUB]) : NULL,
+				subs ? (struct p2_sub *)(b + off[SUB]) : NULL,
 				(struct p2_sub_rec *)(b + off[SREC]),
 				(uint32_t *)(b + off[NSUB]));
 		if (timing)
@@ -686,8 +689,25 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 			e = cudaGetLastError();
 			if (timing)
 				cudaEventRecord(ev[3], d->stream);
-			if (e == cudaSuccess)
+			if (e == cudaSuccess && subs)
 				e = p2_resident_samples(d, a, g);
+			if (e == cudaSuccess && whole) {
+				struct p2_oc_samples o;
+				memset(&o, 0, sizeof o);
+				o.ndet = a.ndet;
+				o.C = a.C;
+				o.T = a.T;
+				o.keep = a.keep;
+				o.passes = (const struct phase2_pass *)(b +
+					off[PASS]);
+				o.npc = npc;
+				o.recs = (const struct phase2_rot_rec *)(b +
+					off[REC]);
+				o.widx = a.widx;
+				o.wval = a.wval;
+				o.gout = a.gout;
+				e = p2_onchip_samples(d, o, g);
+			}
 			if (timing)
 				cudaEventRecord(ev[4], d->stream);
 			d->launches += 3 + (job->depth != 0);
