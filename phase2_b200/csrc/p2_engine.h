@@ -252,11 +252,11 @@ bool p2_resident_samples_ok(const struct p2_dev *d, int form);
 cudaError_t p2_resident_samples(struct p2_dev *d, struct p2_res_samples a,
 	uint32_t g);
 
-/* onchip.cu: the same for many samples, a block each, by
- * whole passes: sample s's passes of chunk c are passes[s * T + c *
+/* onchip.cu: the same for launches of g samples, 2^lb blocks each, by whole
+ * passes: sample s's passes of chunk c are passes[s * T + c *
  * P2_QUEUE_FLUSH ..], npc[s * C + c] of them, their rot_off into recs. */
 struct p2_oc_samples {
-	uint32_t nqb, ndet, C;
+	uint32_t nqb, lb, ndet, C;
 	uint64_t T, keep;
 	const struct phase2_pass *passes;
 	const uint32_t *npc;
@@ -266,7 +266,7 @@ struct p2_oc_samples {
 	double2 *gout;
 	void *state;
 };
-bool p2_onchip_samples_ok(const struct p2_dev *d, int form, uint64_t samples);
+bool p2_onchip_samples_ok(const struct p2_dev *d, int form, uint64_t g);
 cudaError_t p2_onchip_samples(struct p2_dev *d, struct p2_oc_samples a,
 	uint32_t g);
 

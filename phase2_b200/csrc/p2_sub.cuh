@@ -11,54 +11,18 @@
 #define P2_ROT_GROUP 4
 #define P2_LIFT_GROUP 4
 #include "p2_kernels.cuh"
+#include "p2_cluster.cuh"
 #include "sub_core.h"
 
 #define P2_RES_SLOTS (1 << P2_SUB_SPAN)
 
-/* ---- shared memory of the cluster --------------------------------------- */
+/* ---- slots ---------------------------------------------------------------- */
 
 template <bool CL>
 __device__ __forceinline__ uint32_t p2_res_addr(uint32_t base, uint32_t pos,
 	uint32_t kc)
 {
-	uint32_t a = base + ((pos & ((1u << kc) - 1u)) << 4);
-	if constexpr (CL) {
-		const uint32_t rank = pos >> kc;
-		asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a)
-			: "r"(a), "r"(rank));
-	}
-	return a;
-}
-
-template <bool CL>
-__device__ __forceinline__ void p2_res_ld(uint32_t a, double &re, double &im)
-{
-	if constexpr (CL)
-		asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
-			: "=d"(re), "=d"(im) : "r"(a) : "memory");
-	else
-		asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
-			: "=d"(re), "=d"(im) : "r"(a) : "memory");
-}
-
-template <bool CL>
-__device__ __forceinline__ void p2_res_st(uint32_t a, double re, double im)
-{
-	if constexpr (CL)
-		asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};"
-			:: "r"(a), "d"(re), "d"(im) : "memory");
-	else
-		asm volatile("st.shared.v2.f64 [%0], {%1, %2};"
-			:: "r"(a), "d"(re), "d"(im) : "memory");
-}
-
-template <bool CL> __device__ __forceinline__ void p2_res_barrier()
-{
-	if constexpr (CL)
-		asm volatile("barrier.cluster.arrive.release.aligned;\n"
-			     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-	else
-		__syncthreads();
+	return p2_res_map<CL>(base, pos << 4, kc + 4);
 }
 
 /* The rotation (key) on a coset of 8 slots: the exact FP64 update, or the

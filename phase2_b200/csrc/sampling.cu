@@ -472,7 +472,7 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		R = 1;
 	const uint32_t C = (uint32_t)((T + P2_QUEUE_FLUSH - 1) / P2_QUEUE_FLUSH);
 	/* registers that fit on chip: no state copies, no persistent kernel */
-	const bool whole = T > 0 && p2_onchip_samples_ok(d, job->form, samples);
+	const bool whole = T > 0 && p2_onchip_samples_ok(d, job->form, G);
 	const bool subs = T > 0 && !whole &&
 		p2_resident_samples_ok(d, job->form);
 	const bool res = whole || subs;

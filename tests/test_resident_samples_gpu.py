@@ -34,7 +34,8 @@ def _both(kind, prec, *args):
 @pytest.mark.parametrize("prec", [p2.PREC_FP64, p2.PREC_FP32])
 @pytest.mark.parametrize("n,samples,depth", [
     (4, 1, 5), (10, 90, 40), (11, 3, 9000), (12, 1, 70), (12, 80, 60),
-    (13, 9, 60), (13, 20, 60), (13, 75, 20), (14, 2, 60), (14, 40, 60)])
+    (13, 9, 60), (13, 20, 60), (13, 75, 20), (14, 2, 60), (14, 20, 60), (14, 40, 60),
+    (14, 80, 20)])
 def test_qdrift(n, samples, depth, prec):
     t = workloads.jw_terms(n, 50, seed=n + samples)
     # a determinant written twice: the later value holds
