@@ -20,8 +20,10 @@
  * __dmul_rn/__dadd_rn, never fused, so every amplitude is bit-identical to
  * the reference CPU update a_i <- c a_i + i conj(s z) a_j
  * (phase2/qreg_qreg.c:149-160).  FP32 state: each pair is rotated by three
- * in-place shears (the lifted form), in FP32 FMAs (k_pass_lift32, the
- * default) or in FP64 with one rounding to FP32 per pass (k_pass_lift).
+ * in-place shears (the lifted form), in FP32 FMAs (k_pass_lift32) or in
+ * FP64 with one rounding to FP32 per pass (k_pass_lift); by default each
+ * coset by its largest amplitude from 24 qubits up (k_pass_lift32h), FP64
+ * below.
  *
  * Other kernels: gather/scatter of a few amplitudes (overlap, state prep),
  * and a two-stage FP64 sum of squares / inner product (warp-shuffle tree
@@ -30,7 +32,9 @@
  *
  * The device helpers these kernels share live in p2_kernels.cuh; the
  * persistent kernel is in batch.cu, device sampling in sampling.cu and
- * sweeps in sweep.cu.
+ * sweeps in sweep.cu.  A flush runs on other kernels where these leave the
+ * chip idle (p2d_run): resident.cu up to 14 qubits, split.cu from 15 to 19,
+ * tile.cu for FP64 registers of 20 qubits up with few rotations a pass.
  */
 #include <cuda_runtime.h>
 
