@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(P2_TPB, M >= 5 ? 3 : p2_min_blocks(M))
 		o.s = in.s;
 		o.z = in.z;
 		o.sm = in.smask;
-		o.key = ((uint32_t)in.U << 1) | in.odd;
+		o.key = ((uint32_t)in.U << 1) | in.odd |
+			p2_lift_sv(in.U, in.smask, M) << 6;
 		srec[r] = o;
 	}
 	__syncthreads();
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(P2_TPB, M >= 5 ? 3 : p2_min_blocks(M))
 		for (uint32_t r = 0; r < nrot; ++r) {
 			const struct p2_lift_rec q = srec[r];
 			const uint32_t sm = q.sm ^ (0u - p2_parity(x & (IT)q.z));
-			p2_apply_lift<M>(q.key, re, im, q.t, q.s, sm);
+			p2_apply_lift_sv<M>(q.key, re, im, q.t, q.s, sm);
 		}
 		if (neg) {
 #pragma unroll

@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(P2_LB_TPB, p2_lb_blocks(M))
 		o.s = in.s;
 		o.z = in.z;
 		o.sm = in.smask;
-		o.key = ((uint32_t)in.U << 1) | in.odd;
+		o.key = ((uint32_t)in.U << 1) | in.odd |
+			p2_lift_sv(in.U, in.smask, M) << 6;
 		srec[r] = o;
 	}
 	const uint32_t bar0 = p2_saddr(&sbar[wid][0]);
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(P2_LB_TPB, p2_lb_blocks(M))
 			const struct p2_lift_rec q = srec[r];
 			const uint32_t sm =
 				q.sm ^ (0u - p2_parity(x & (uint32_t)q.z));
-			p2_apply_lift<M>(q.key, re, im, q.t, q.s, sm);
+			p2_apply_lift_sv<M>(q.key, re, im, q.t, q.s, sm);
 		}
 		if (neg)
 			p2_lb_store<M, true>(st, x, pb, re, im);
@@ -285,7 +286,8 @@ __global__ void __launch_bounds__(P2_LB_TPB, MINB)
 		o.s = in.s;
 		o.z = in.z;
 		o.sm = in.smask;
-		o.key = ((uint32_t)in.U << 1) | in.odd;
+		o.key = ((uint32_t)in.U << 1) | in.odd |
+			p2_lift_sv(in.U, in.smask, M) << 6;
 		srec[r] = o;
 	}
 	__syncthreads();
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(P2_LB_TPB, MINB)
 			const struct p2_lift_rec q = srec[r];
 			const uint32_t sm =
 				q.sm ^ (0u - p2_parity(x & (uint32_t)q.z));
-			p2_apply_lift<M>(q.key, re, im, q.t, q.s, sm);
+			p2_apply_lift_sv<M>(q.key, re, im, q.t, q.s, sm);
 		}
 		if (neg)
 			p2_lb_store<M, true>(st, x, pb, re, im);

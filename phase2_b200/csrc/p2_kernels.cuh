@@ -296,6 +296,16 @@ __device__ __forceinline__ void p2_prefetch(double2 *stage, const double2 *st,
  * anew cost 4-17 % of the rotation, most where few warps share a
  * scheduler).  Rounding is symmetric under negation, so this gives the same
  * bits as flipping the partner's sign around the shears.
+ *
+ * SB > 0: the sign's changes along the walk's first SB bits are template
+ * arguments (SV), so 2^SB pairs share one copy of the coefficients, negated
+ * as operands, and the walk XORs once a group: of 250 instructions a
+ * rotation at M = 5, 96 of them FMAs, the signs were 64.  SB = 2 is four
+ * times the cases, for the kernels that run one pass a launch (1e12
+ * rotations x amplitudes a second at 20 / 23 qubits, SB = 0, 1, 2: 5.5
+ * draws a pass 0.93 / 1.64, 0.97 / 1.79, 1.00 / 1.87; 13-17 strings a pass
+ * 1.45 / 2.39, 1.53 / 2.65, 1.51 / 2.75; 250 a pass 2.05 / 2.28, 2.36 /
+ * 2.68, 2.57 / 3.05).
  * U = 0 (the string is diagonal on the coset, and then odd = 1) is the
  * phase c + i sigma s, applied to (re, im) by the same three shears.
  *
@@ -307,6 +317,7 @@ __device__ __forceinline__ void p2_prefetch(double2 *stage, const double2 *st,
 #ifndef P2_LIFT_GROUP
 #define P2_LIFT_GROUP 2
 #endif
+#define P2_LIFT_SB 2
 #ifndef P2_LIFT32_GROUP
 #define P2_LIFT32_GROUP 4
 #endif
@@ -323,7 +334,44 @@ __host__ __device__ constexpr int p2_gray_bit(int i)
 	return i & 1 ? 0 : i & 2 ? 1 : i & 4 ? 2 : i & 8 ? 3 : 4;
 }
 
-template <int M, int U, int ODD>
+/* Step i of a walk whose low B bits count and whose others step in Gray
+ * code order. */
+__host__ __device__ constexpr int p2_walk(int i, int B)
+{
+	return p2_gray(i >> B) << B | (i & ((1 << B) - 1));
+}
+
+/* st[j], ss[j] of group g: with B = 0 the sign changes from step to step;
+ * else from group to group, and inside one by bits of SV. */
+#define P2_LIFT_SIGNS(B, BIT)                                                  \
+	if constexpr (B == 0) {                                                \
+		_Pragma("unroll") for (int j = 0; j < G; ++j)                  \
+		{                                                              \
+			if (g + j > 0) {                                       \
+				const int b = p2_gray_bit(g + j);              \
+				const uint32_t f = mk[BIT];                    \
+				t0 = p2_sgn(t0, f);                            \
+				s0 = p2_sgn(s0, f);                            \
+			}                                                      \
+			st[j] = t0;                                            \
+			ss[j] = s0;                                            \
+		}                                                              \
+	} else {                                                               \
+		if (g > 0) {                                                   \
+			const int b = p2_gray_bit(g >> B) + B;                 \
+			const uint32_t f = mk[BIT];                            \
+			t0 = p2_sgn(t0, f);                                    \
+			s0 = p2_sgn(s0, f);                                    \
+		}                                                              \
+		_Pragma("unroll") for (int j = 0; j < G; ++j)                  \
+		{                                                              \
+			const bool n = ((j & SV & 1) ^ (j & SV) >> 1) & 1;     \
+			st[j] = n ? -t0 : t0;                                  \
+			ss[j] = n ? -s0 : s0;                                  \
+		}                                                              \
+	}
+
+template <int M, int U, int ODD, int SB = 0, int SV = 0>
 __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 	double (&im)[1 << M], double t, double s, uint32_t sm)
 {
@@ -334,35 +382,28 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 		mk[k] = ((sm << (31 - (1 << k))) ^ (sm << 31)) & 0x80000000u;
 	double t0 = p2_sgn(t, sm << 31), s0 = p2_sgn(s, sm << 31);
 	if constexpr (U == 0) {
+		constexpr int B = SB < M ? SB : M;
 		constexpr int S = 1 << M;
-		constexpr int G = S < P2_LIFT_GROUP ? S : P2_LIFT_GROUP;
+		constexpr int G = B > 0 ? 1 << B
+			: S < P2_LIFT_GROUP ? S : P2_LIFT_GROUP;
 #pragma unroll
 		for (int g = 0; g < S; g += G) {
 			double st[G], ss[G];
-#pragma unroll
-			for (int j = 0; j < G; ++j) {
-				if (g + j > 0) {
-					const uint32_t f = mk[p2_gray_bit(g + j)];
-					t0 = p2_sgn(t0, f);
-					s0 = p2_sgn(s0, f);
-				}
-				st[j] = t0;
-				ss[j] = s0;
-			}
+			P2_LIFT_SIGNS(B, b)
 			if constexpr (ODD) {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_gray(g + j);
+					const int u = p2_walk(g + j, B);
 					re[u] = fma(-st[j], im[u], re[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_gray(g + j);
+					const int u = p2_walk(g + j, B);
 					im[u] = fma(ss[j], re[u], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_gray(g + j);
+					const int u = p2_walk(g + j, B);
 					re[u] = fma(-st[j], im[u], re[u]);
 				}
 			} else {
@@ -370,7 +411,7 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 				 * that is diagonal on the coset never has it */
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_gray(g + j);
+					const int u = p2_walk(g + j, B);
 					const double k = ss[j] + fma(-t, s, 1.0);
 					re[u] *= k;
 					im[u] *= k;
@@ -380,39 +421,31 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 	} else {
 		constexpr int H = p2_hibit(U);
 		constexpr int NP = 1 << (M - 1);
-		constexpr int G = NP < P2_LIFT_GROUP ? NP : P2_LIFT_GROUP;
+		constexpr int B = SB < M - 1 ? SB : M - 1;
+		constexpr int G = B > 0 ? 1 << B
+			: NP < P2_LIFT_GROUP ? NP : P2_LIFT_GROUP;
 #pragma unroll
 		for (int g = 0; g < NP; g += G) {
 			double st[G], ss[G];
-#pragma unroll
-			for (int j = 0; j < G; ++j) {
-				if (g + j > 0) {
-					const int b = p2_gray_bit(g + j);
-					const uint32_t f = mk[b < H ? b : b + 1];
-					t0 = p2_sgn(t0, f);
-					s0 = p2_sgn(s0, f);
-				}
-				st[j] = t0;
-				ss[j] = s0;
-			}
+			P2_LIFT_SIGNS(B, b < H ? b : b + 1)
 			if constexpr (ODD) {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[u] = fma(-st[j], im[w], re[u]);
 					im[u] = fma(st[j], re[w], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[w] = fma(-ss[j], im[u], re[w]);
 					im[w] = fma(ss[j], re[u], im[w]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[u] = fma(-st[j], im[w], re[u]);
 					im[u] = fma(st[j], re[w], im[u]);
@@ -420,21 +453,21 @@ __device__ __forceinline__ void p2_rot_lift(double (&re)[1 << M],
 			} else {
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[u] = fma(st[j], re[w], re[u]);
 					im[u] = fma(st[j], im[w], im[u]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[w] = fma(-ss[j], re[u], re[w]);
 					im[w] = fma(-ss[j], im[u], im[w]);
 				}
 #pragma unroll
 				for (int j = 0; j < G; ++j) {
-					const int u = p2_ins0(p2_gray(g + j), H),
+					const int u = p2_ins0(p2_walk(g + j, B), H),
 						  w = u ^ U;
 					re[u] = fma(st[j], re[w], re[u]);
 					im[u] = fma(st[j], im[w], im[u]);
@@ -478,6 +511,48 @@ __device__ __forceinline__ void p2_apply_lift(uint32_t key,
 	}
 }
 #undef P2_CASE_L
+
+/* Bits of SV for a rotation: the sign's change along the first two bits of
+ * the walk over its pairs (slots, when it is diagonal on the coset). */
+__device__ __forceinline__ uint32_t p2_lift_sv(uint32_t U, uint32_t sm, int M)
+{
+	const int H = U ? 31 - __clz((int)U) : M;
+	const int n = U ? M - 1 : M;
+	uint32_t v = 0;
+	for (int k = 0; k < P2_LIFT_SB && k < n; ++k)
+		v |= ((sm >> (1 << (k < H ? k : k + 1)) ^ sm) & 1u) << k;
+	return v;
+}
+
+#define P2_CASE_LS(K, V)                                                       \
+	case (K) | (V) << 6:                                                   \
+		if constexpr ((K) < (2 << M))                                  \
+			p2_rot_lift<M, ((K) >> 1), ((K)&1), P2_LIFT_SB, (V)>(  \
+				re, im, t, s, sm);                             \
+		break;
+#define P2_CASE_LS8(K, V)                                                      \
+	P2_CASE_LS(K, V) P2_CASE_LS(K + 1, V) P2_CASE_LS(K + 2, V)                \
+	P2_CASE_LS(K + 3, V) P2_CASE_LS(K + 4, V) P2_CASE_LS(K + 5, V)            \
+	P2_CASE_LS(K + 6, V) P2_CASE_LS(K + 7, V)
+#define P2_CASE_LS64(V)                                                        \
+	P2_CASE_LS8(0, V) P2_CASE_LS8(8, V) P2_CASE_LS8(16, V) P2_CASE_LS8(24, V)  \
+	P2_CASE_LS8(32, V) P2_CASE_LS8(40, V) P2_CASE_LS8(48, V) P2_CASE_LS8(56, V)
+
+/* key = SV << 6 | U << 1 | odd */
+template <int M>
+__device__ __forceinline__ void p2_apply_lift_sv(uint32_t key,
+	double (&re)[1 << M], double (&im)[1 << M], double t, double s,
+	uint32_t sm)
+{
+	switch (key) {
+		P2_CASE_LS64(0) P2_CASE_LS64(1) P2_CASE_LS64(2) P2_CASE_LS64(3)
+	default:
+		break;
+	}
+}
+#undef P2_CASE_LS
+#undef P2_CASE_LS8
+#undef P2_CASE_LS64
 
 /* A lifted record as the kernel reads it from shared memory. */
 struct p2_lift_rec {
