@@ -772,7 +772,8 @@ static struct p2_dev *shells[P2_SHELLS];
 static int nshells;
 
 /* A number that differs between a device's contexts (a device reset makes
- * a new one, in which kept handles mean nothing); 0 where it is unknown. */
+ * a new one, in which kept handles mean nothing); 0 where it is unknown or
+ * the thread has no context. */
 static uint64_t context_id(void)
 {
 	typedef int (*get_id)(void *, unsigned long long *);
@@ -791,6 +792,20 @@ static uint64_t context_id(void)
 	unsigned long long id = 0;
 	if (!fn || fn(NULL, &id) != 0)
 		return 0;
+	return id;
+}
+
+/* The same, after making the device's context current: a thread's first
+ * call, or the first after a reset, would find none, and the shells of two
+ * such contexts would share the number 0. */
+static uint64_t context_use(void)
+{
+	uint64_t id = context_id();
+	if (id == 0) {
+		if (cudaFree(NULL) == cudaSuccess)
+			id = context_id();
+		cudaGetLastError();
+	}
 	return id;
 }
 
@@ -858,7 +873,7 @@ fail:
 /* A shell of device `dev` in the current context: a kept one or a new one. */
 static struct p2_dev *shell_take(int dev)
 {
-	const uint64_t ctx = context_id();
+	const uint64_t ctx = context_use();
 	struct p2_dev *d = NULL;
 	pthread_mutex_lock(&shell_lock);
 	for (int k = nshells - 1; k >= 0 && !d; k--)
@@ -1276,15 +1291,6 @@ extern "C" int phase2_tune_get(int prec, int span, int *variant, int *per_sm)
 	return 0;
 }
 
-/* Resolved configuration of the prefetch kernel (shared memory opt-in and
- * resident blocks per SM), once per instantiation. */
-struct p2_kcfg {
-	int ready;
-	int tpb;
-	size_t smem;
-	int per_sm;
-};
-
 /* One FP64 pass: direct (variant 0) or prefetch (variant 1) kernel. */
 template <int M>
 static int launch_pass_t(struct p2_dev *d, const struct phase2_pass &p,
@@ -1301,26 +1307,27 @@ static int launch_pass_t(struct p2_dev *d, const struct phase2_pass &p,
 			"pass launch");
 		return 0;
 	}
-	static struct p2_kcfg cfg;
-	if (!cfg.ready) {
-		cfg.tpb = p2_tpb(M);
-		cfg.smem = 2 * ((size_t)1 << M) * cfg.tpb * sizeof(double2);
+	const int tpb = p2_tpb(M);
+	const size_t smem = 2 * ((size_t)1 << M) * tpb * sizeof(double2);
+	static uint64_t done;
+	unsigned most; /* resident blocks per SM */
+	if (!p2_done(&done, d->context, &most)) {
 		CUDA_OK(cudaFuncSetAttribute(k_pass_pf<M>,
 				cudaFuncAttributeMaxDynamicSharedMemorySize,
-				(int)cfg.smem),
+				(int)smem),
 			"pass kernel shared memory");
-		int per_sm = 0;
-		CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
-				k_pass_pf<M>, cfg.tpb, cfg.smem),
+		int n = 0;
+		CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n,
+				k_pass_pf<M>, tpb, smem),
 			"pass kernel occupancy");
-		cfg.per_sm = per_sm > 0 ? per_sm : 1;
-		cfg.ready = 1;
+		most = n > 0 ? (unsigned)n : 1;
+		p2_set_done(&done, d->context, most);
 	}
-	const unsigned per_sm = te.per_sm && te.per_sm < cfg.per_sm
+	const unsigned per_sm = te.per_sm && (unsigned)te.per_sm < most
 		? (unsigned)te.per_sm
-		: (unsigned)cfg.per_sm;
-	const unsigned grid = grid_for(d, nrep, (unsigned)cfg.tpb, per_sm);
-	CUDA_OK(p2_launch(k_pass_pf<M>, grid, cfg.tpb, cfg.smem,
+		: most;
+	const unsigned grid = grid_for(d, nrep, (unsigned)tpb, per_sm);
+	CUDA_OK(p2_launch(k_pass_pf<M>, grid, tpb, smem,
 				d->stream, sv, nrep, p, recs),
 			"pass launch");
 	return 0;
@@ -1907,14 +1914,16 @@ extern "C" void *p2d_stream(const struct p2_dev *d)
 
 cudaError_t p2_scratch_alloc(void **p, size_t bytes, cudaStream_t stream)
 {
-	/* once per device (devices 0..63): keep freed memory of up to a
+	/* once per context (devices 0..63): keep freed memory of up to a
 	 * sixteenth of the device's in its default pool (11 GiB of 180; mapping
 	 * and unmapping a register's 8 GiB took 88 ms a run, as long as 30
 	 * passes over it); p2d_release gives it back */
-	static uint64_t pool_ready;
+	static uint64_t pool_done[64];
+	const uint64_t ctx = context_use();
+	unsigned ok;
 	int dev = 0;
 	if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 &&
-		!(pool_ready >> dev & 1)) {
+		!p2_done(&pool_done[dev], ctx, &ok)) {
 		cudaMemPool_t pool;
 		if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
 			uint64_t keep = UINT64_C(1) << 30;
@@ -1926,7 +1935,7 @@ cudaError_t p2_scratch_alloc(void **p, size_t bytes, cudaStream_t stream)
 				cudaMemPoolAttrReleaseThreshold, &keep);
 		}
 		cudaGetLastError(); /* a pool call's failure is not the caller's */
-		pool_ready |= UINT64_C(1) << dev;
+		p2_set_done(&pool_done[dev], ctx, 1);
 	}
 	return cudaMallocAsync(p, bytes, stream);
 }

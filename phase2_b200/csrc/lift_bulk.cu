@@ -372,11 +372,6 @@ __global__ void __launch_bounds__(P2_LB_TPB, MINB)
 	p2_cp_wait<0>();
 }
 
-struct p2_lb_cfg {
-	int ready;
-	int per_sm;
-};
-
 /* Grid of a staged kernel: resident blocks per SM (occupancy, capped),
  * at most one block per four warp-cosets. */
 static unsigned lb_grid(const struct p2_dev *d, int per_sm_occ,
@@ -396,9 +391,10 @@ template <int M, int MINB>
 static int pf_launch_t(struct p2_dev *d, const struct phase2_pass *p,
 	const struct phase2_rot_rec *recs, unsigned per_sm_cap)
 {
-	static struct p2_lb_cfg cfg;
+	static uint64_t done;
+	unsigned per_sm;
 	const unsigned smem = p2_lb_smem(M);
-	if (!cfg.ready) {
+	if (!p2_done(&done, d->context, &per_sm)) {
 		CUDA_OK(cudaFuncSetAttribute(k_pass_lift_pf<M, MINB>,
 				cudaFuncAttributeMaxDynamicSharedMemorySize,
 				(int)smem),
@@ -407,12 +403,12 @@ static int pf_launch_t(struct p2_dev *d, const struct phase2_pass *p,
 		CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n,
 				k_pass_lift_pf<M, MINB>, P2_LB_TPB, smem),
 			"staged pass occupancy");
-		cfg.per_sm = n > 0 ? n : 1;
-		cfg.ready = 1;
+		per_sm = n > 0 ? (unsigned)n : 1;
+		p2_set_done(&done, d->context, per_sm);
 	}
 	const uint32_t nwc = (uint32_t)((d->namp >> M) >> 5);
 	CUDA_OK(p2_launch(k_pass_lift_pf<M, MINB>,
-			lb_grid(d, cfg.per_sm, per_sm_cap, nwc), P2_LB_TPB, smem,
+			lb_grid(d, (int)per_sm, per_sm_cap, nwc), P2_LB_TPB, smem,
 			d->stream, (float2 *)d->state, nwc, *p, recs),
 		"staged pass launch");
 	return 1;
@@ -422,9 +418,10 @@ template <int M>
 static int lb_launch_t(struct p2_dev *d, const struct phase2_pass *p,
 	const struct phase2_rot_rec *recs, unsigned per_sm_cap)
 {
-	static struct p2_lb_cfg cfg;
+	static uint64_t done;
+	unsigned per_sm;
 	const unsigned smem = p2_lb_smem(M);
-	if (!cfg.ready) {
+	if (!p2_done(&done, d->context, &per_sm)) {
 		CUDA_OK(cudaFuncSetAttribute(k_pass_lift_bulk<M>,
 				cudaFuncAttributeMaxDynamicSharedMemorySize,
 				(int)smem),
@@ -433,11 +430,11 @@ static int lb_launch_t(struct p2_dev *d, const struct phase2_pass *p,
 		CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n,
 				k_pass_lift_bulk<M>, P2_LB_TPB, smem),
 			"staged pass occupancy");
-		cfg.per_sm = n > 0 ? n : 1;
-		cfg.ready = 1;
+		per_sm = n > 0 ? (unsigned)n : 1;
+		p2_set_done(&done, d->context, per_sm);
 	}
 	const uint32_t nwc = (uint32_t)((d->namp >> M) >> 5);
-	k_pass_lift_bulk<M><<<lb_grid(d, cfg.per_sm, per_sm_cap, nwc),
+	k_pass_lift_bulk<M><<<lb_grid(d, (int)per_sm, per_sm_cap, nwc),
 		P2_LB_TPB, smem, d->stream>>>((float2 *)d->state, nwc, *p,
 		recs, d->d_status);
 	d->status_pending = 1;

@@ -268,20 +268,18 @@ static uint32_t onchip_blocks(const struct p2_dev *d, uint64_t g)
 	return lb;
 }
 
-template <auto F> static bool onchip_ready(void)
+template <auto F> static bool onchip_ready(const struct p2_dev *d)
 {
-	static unsigned ready; /* 1 yes, 2 no */
-	unsigned r = __atomic_load_n(&ready, __ATOMIC_ACQUIRE);
-	if (!r) {
-		r = cudaFuncSetAttribute(F,
-			    cudaFuncAttributeMaxDynamicSharedMemorySize,
-			    (int)P2_OC_SMEM) == cudaSuccess
-			? 1
-			: 2;
+	static uint64_t done;
+	unsigned ok;
+	if (!p2_done(&done, d->context, &ok)) {
+		ok = cudaFuncSetAttribute(F,
+			     cudaFuncAttributeMaxDynamicSharedMemorySize,
+			     (int)P2_OC_SMEM) == cudaSuccess;
 		cudaGetLastError();
-		__atomic_store_n(&ready, r, __ATOMIC_RELEASE);
+		p2_set_done(&done, d->context, ok);
 	}
-	return r == 1;
+	return ok;
 }
 
 /*
@@ -302,12 +300,12 @@ bool p2_onchip_samples_ok(const struct p2_dev *d, int form, uint64_t g)
 	if (d->prec == PHASE2_PREC_FP64)
 		return ((d->nqb == 13 && g >= 16) ||
 			       (d->nqb == 14 && g >= 8)) &&
-			onchip_ready<k_onchip_smp<double2, true>>() &&
-			onchip_ready<k_onchip_smp<double2, false>>();
+			onchip_ready<k_onchip_smp<double2, true>>(d) &&
+			onchip_ready<k_onchip_smp<double2, false>>(d);
 	return ((d->nqb == 12 && g >= 4) || (d->nqb == 13 && g >= 8) ||
 		       d->nqb == 14) &&
-		onchip_ready<k_onchip_smp<float2, true>>() &&
-		onchip_ready<k_onchip_smp<float2, false>>();
+		onchip_ready<k_onchip_smp<float2, true>>(d) &&
+		onchip_ready<k_onchip_smp<float2, false>>(d);
 }
 
 cudaError_t p2_onchip_samples(struct p2_dev *d, struct p2_oc_samples a,

@@ -157,6 +157,26 @@ __device__ __forceinline__ void p2_grid_wait()
 }
 #endif
 
+/*
+ * What is set on a kernel (shared memory, cluster size) belongs to the
+ * device's context, and a device reset makes a new one: a "done" word holds
+ * the context's number (p2_dev.context) above a byte of the answer, so one
+ * of another context counts as unset.
+ */
+static inline bool p2_done(const uint64_t *word, uint64_t context,
+	unsigned *answer)
+{
+	const uint64_t w = __atomic_load_n(word, __ATOMIC_ACQUIRE);
+	*answer = (unsigned)(w & 0x7f);
+	return (w & 0x80) && w >> 8 == context;
+}
+
+static inline void p2_set_done(uint64_t *word, uint64_t context,
+	unsigned answer)
+{
+	__atomic_store_n(word, context << 8 | 0x80 | answer, __ATOMIC_RELEASE);
+}
+
 /* ---- cross-file entry points -------------------------------------------- */
 
 /* engine.cu: transient device buffers of one call (a batch program, the

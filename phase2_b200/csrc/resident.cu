@@ -504,15 +504,16 @@ fail:
 }
 
 /* Largest cluster a kernel can be launched with on this device (blocks of
- * 128 threads and 16 KiB), once per kernel; 0 when it cannot be
+ * 128 threads and 16 KiB), once per kernel and context; 0 when it cannot be
  * configured. */
-template <auto F> static unsigned res_clusters(bool clusters)
+template <auto F>
+static unsigned res_clusters(const struct p2_dev *d, bool clusters)
 {
-	static unsigned most; /* 1 + the answer */
-	unsigned m = __atomic_load_n(&most, __ATOMIC_ACQUIRE);
-	if (m)
-		return m - 1;
-	unsigned best = 0;
+	static uint64_t done;
+	unsigned best;
+	if (p2_done(&done, d->context, &best))
+		return best;
+	best = 0;
 	if (cudaFuncSetAttribute(F, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		    P2_RES_SMEM) == cudaSuccess) {
 		best = 1;
@@ -540,7 +541,7 @@ template <auto F> static unsigned res_clusters(bool clusters)
 		}
 	}
 	cudaGetLastError();
-	__atomic_store_n(&most, best + 1, __ATOMIC_RELEASE);
+	p2_set_done(&done, d->context, best);
 	return best;
 }
 
@@ -557,10 +558,10 @@ bool p2_resident_ok(const struct p2_dev *d, int form)
 		return false;
 	const uint32_t lb = res_log_blocks(d->nqb);
 	const unsigned most = d->prec == PHASE2_PREC_FP64
-		? (lb ? res_clusters<k_resident<double2, false, true>>(true)
-		      : res_clusters<k_resident<double2, false, false>>(false))
-		: (lb ? res_clusters<k_resident<float2, true, true>>(true)
-		      : res_clusters<k_resident<float2, true, false>>(false));
+		? (lb ? res_clusters<k_resident<double2, false, true>>(d, true)
+		      : res_clusters<k_resident<double2, false, false>>(d, false))
+		: (lb ? res_clusters<k_resident<float2, true, true>>(d, true)
+		      : res_clusters<k_resident<float2, true, false>>(d, false));
 	return most >= (1u << lb);
 }
 
@@ -648,14 +649,14 @@ bool p2_resident_samples_ok(const struct p2_dev *d, int form)
 	/* both kernels: the number of samples chooses between them */
 	const unsigned need = 1u << res_log_blocks(d->nqb);
 	return d->prec == PHASE2_PREC_FP64
-		? res_clusters<k_resident_smp<double2, false, true>>(true) >=
+		? res_clusters<k_resident_smp<double2, false, true>>(d, true) >=
 				need &&
 			res_clusters<k_resident_smp<double2, false, false>>(
-				false) >= 1
-		: res_clusters<k_resident_smp<float2, true, true>>(true) >=
+				d, false) >= 1
+		: res_clusters<k_resident_smp<float2, true, true>>(d, true) >=
 				need &&
 			res_clusters<k_resident_smp<float2, true, false>>(
-				false) >= 1;
+				d, false) >= 1;
 }
 
 template <typename ST, bool X>
@@ -686,12 +687,12 @@ bool p2_resident_prog_ok(const struct p2_dev *d, int form)
 		return false;
 	/* any width's clusters: the batch's widest register chooses them */
 	return d->prec == PHASE2_PREC_FP64
-		? res_clusters<k_resident_prog<double2, false, true>>(true) >= 16 &&
+		? res_clusters<k_resident_prog<double2, false, true>>(d, true) >= 16 &&
 			res_clusters<k_resident_prog<double2, false, false>>(
-				false) >= 1
-		: res_clusters<k_resident_prog<float2, true, true>>(true) >= 16 &&
+				d, false) >= 1
+		: res_clusters<k_resident_prog<float2, true, true>>(d, true) >= 16 &&
 			res_clusters<k_resident_prog<float2, true, false>>(
-				false) >= 1;
+				d, false) >= 1;
 }
 
 template <typename ST, bool X>

@@ -158,14 +158,15 @@ template <typename ST, bool X, int M>
 static cudaError_t split_launch_m(struct p2_dev *d, const struct p2_split_pass &sp,
 	const struct p2_sub *subs, const struct p2_sub_rec *recs)
 {
-	static int ready;
-	if (!__atomic_load_n(&ready, __ATOMIC_ACQUIRE)) {
+	static uint64_t done;
+	unsigned ok;
+	if (!p2_done(&done, d->context, &ok)) {
 		const cudaError_t e = cudaFuncSetAttribute(k_pass_split<ST, X, M>,
 			cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)P2_SPLIT_SMEM);
 		if (e != cudaSuccess)
 			return e;
-		__atomic_store_n(&ready, 1, __ATOMIC_RELEASE);
+		p2_set_done(&done, d->context, 1);
 	}
 	return p2_launch(k_pass_split<ST, X, M>,
 		(unsigned)(d->namp >> P2_SPLIT_BITS), P2_SPLIT_TPB,

@@ -370,15 +370,16 @@ static int launch_sweep(struct p2_dev *d, const struct p2_sweep &sw,
 	const size_t smem = ((size_t)8 << tl) +
 		(size_t)sw.nrec * sizeof(struct p2_lift32_rec) +
 		((size_t)4 << sw.k);
-	static int smem_set;
-	if (!smem_set) {
+	static uint64_t done;
+	unsigned ok;
+	if (!p2_done(&done, d->context, &ok)) {
 		CUDA_OK(cudaFuncSetAttribute(k_sweep32,
 				cudaFuncAttributeMaxDynamicSharedMemorySize,
 				(int)(((size_t)8 << P2_SW_MAXTILE) +
 					P2_SW_MAXREC * sizeof(struct p2_lift32_rec) +
 					((size_t)4 << P2_SW_MAXK))),
 			"sweep kernel shared memory");
-		smem_set = 1;
+		p2_set_done(&done, d->context, 1);
 	}
 	const uint32_t ntiles = (uint32_t)(d->namp >> tl);
 	uint32_t grid = (uint32_t)d->sm_count * 2;

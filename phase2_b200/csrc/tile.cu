@@ -232,9 +232,10 @@ int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
 	if (!g)
 		return -1;
 	d->graph_replays += hit;
-	static int per_sm;
-	int n = __atomic_load_n(&per_sm, __ATOMIC_ACQUIRE);
-	if (!n) {
+	static uint64_t done;
+	unsigned per_sm;
+	if (!p2_done(&done, d->context, &per_sm)) {
+		int n = 0;
 		CUDA_OK(cudaFuncSetAttribute(k_tile,
 				cudaFuncAttributeMaxDynamicSharedMemorySize,
 				(int)P2_TILE_BYTES),
@@ -242,11 +243,11 @@ int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
 		CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile,
 				P2_TILE_TPB, P2_TILE_BYTES),
 			"tile kernel occupancy");
-		n = n > 0 ? n : 1;
-		__atomic_store_n(&per_sm, n, __ATOMIC_RELEASE);
+		per_sm = n > 0 ? (unsigned)n : 1;
+		p2_set_done(&done, d->context, per_sm);
 	}
 	const uint64_t ntile = d->namp >> P2_TILE_BITS;
-	uint64_t grid = (uint64_t)d->sm_count * (unsigned)n;
+	uint64_t grid = (uint64_t)d->sm_count * per_sm;
 	if (grid > ntile)
 		grid = ntile;
 	if (d->timing)
