@@ -761,8 +761,9 @@ static int io_reserve(struct p2_dev *d, size_t n)
  * Creating and freeing them costs 3 ms where no other register keeps the
  * allocator's blocks alive (a whole 10-qubit run computes for 0.1 ms), so
  * a destroyed register leaves them for the next one: at most
- * P2_SHELLS of them, each holding at most P2_SHELL_BYTES of buffers, per
- * context, given back by p2d_release (world_free).
+ * P2_SHELLS of them, each holding at most P2_SHELL_BYTES of buffers, given
+ * back by p2d_release (world_free); registers destroyed after it keep
+ * nothing until the next one is created.
  */
 #define P2_SHELLS 32
 #define P2_SHELL_BYTES ((size_t)2 << 20)
@@ -770,6 +771,7 @@ static int io_reserve(struct p2_dev *d, size_t n)
 static pthread_mutex_t shell_lock = PTHREAD_MUTEX_INITIALIZER;
 static struct p2_dev *shells[P2_SHELLS];
 static int nshells;
+static int shells_closed;
 
 /* A number that differs between a device's contexts (a device reset makes
  * a new one, in which kept handles mean nothing); 0 where it is unknown or
@@ -876,6 +878,7 @@ static struct p2_dev *shell_take(int dev)
 	const uint64_t ctx = context_use();
 	struct p2_dev *d = NULL;
 	pthread_mutex_lock(&shell_lock);
+	shells_closed = 0;
 	for (int k = nshells - 1; k >= 0 && !d; k--)
 		if (shells[k]->device == dev && shells[k]->context == ctx) {
 			d = shells[k];
@@ -885,9 +888,25 @@ static struct p2_dev *shell_take(int dev)
 	return d ? d : shell_make(dev, ctx);
 }
 
+/* Devices whose default pool keeps freed memory (p2_scratch_alloc). */
+static uint64_t pool_done[64];
+
+/* Give the freed memory in these pools back. */
+static void pool_trim(void)
+{
+	for (int dev = 0; dev < 64; dev++) {
+		cudaMemPool_t pool;
+		if (__atomic_load_n(&pool_done[dev], __ATOMIC_ACQUIRE) &&
+			cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+			cudaMemPoolTrimTo(pool, 0);
+	}
+	cudaGetLastError();
+}
+
 /* Keep a register's shell (its state and plans are gone) or free it. */
 static void shell_give(struct p2_dev *d)
 {
+	bool closed = false;
 	/* a register whose stream reports an error, or whose status word was
 	 * never read, is not reused */
 	bool keep = cudaStreamSynchronize(d->stream) == cudaSuccess &&
@@ -925,36 +944,40 @@ static void shell_give(struct p2_dev *d)
 		fresh.t0 = d->t0;
 		fresh.t1 = d->t1;
 		*d = fresh;
-		pthread_mutex_lock(&shell_lock);
-		keep = nshells < P2_SHELLS;
-		if (keep)
-			shells[nshells++] = d;
-		pthread_mutex_unlock(&shell_lock);
 	}
+	pthread_mutex_lock(&shell_lock);
+	closed = shells_closed;
+	keep = keep && !closed && nshells < P2_SHELLS;
+	if (keep)
+		shells[nshells++] = d;
+	pthread_mutex_unlock(&shell_lock);
 	if (!keep)
 		shell_free(d);
+	if (closed)
+		pool_trim();
 }
 
 extern "C" void p2d_release(void)
 {
-	const uint64_t ctx = context_id();
-	pthread_mutex_lock(&shell_lock);
-	int left = 0;
-	for (int k = 0; k < nshells; k++) {
-		/* of another context: its handles are not this one's to free */
-		if (shells[k]->context == ctx)
-			shell_free(shells[k]);
-		else
-			shells[left++] = shells[k];
-	}
-	nshells = left;
-	pthread_mutex_unlock(&shell_lock);
 	int dev = 0;
-	cudaMemPool_t pool;
-	if (cudaGetDevice(&dev) == cudaSuccess &&
-		cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
-		cudaMemPoolTrimTo(pool, 0);
-	cudaGetLastError();
+	pthread_mutex_lock(&shell_lock);
+	const bool back = nshells > 0 && cudaGetDevice(&dev) == cudaSuccess;
+	shells_closed = 1;
+	for (int k = 0; k < nshells; k++) {
+		struct p2_dev *const d = shells[k];
+		if (cudaSetDevice(d->device) == cudaSuccess &&
+			context_use() == d->context) {
+			shell_free(d);
+		} else {
+			/* the handles went with their context */
+			free(d);
+		}
+	}
+	nshells = 0;
+	pthread_mutex_unlock(&shell_lock);
+	if (back)
+		cudaSetDevice(dev);
+	pool_trim();
 }
 
 extern "C" struct p2_dev *p2d_create(uint32_t nqb, int prec)
@@ -1918,7 +1941,6 @@ cudaError_t p2_scratch_alloc(void **p, size_t bytes, cudaStream_t stream)
 	 * sixteenth of the device's in its default pool (11 GiB of 180; mapping
 	 * and unmapping a register's 8 GiB took 88 ms a run, as long as 30
 	 * passes over it); p2d_release gives it back */
-	static uint64_t pool_done[64];
 	const uint64_t ctx = context_use();
 	unsigned ok;
 	int dev = 0;
