@@ -33,10 +33,12 @@ void p2_settings_from_env(void);
  * rotations (q) and amplitude writes (w*).  At most one of them is
  * non-empty: queuing into one drains the other first.  Reads drain both.
  * Registers of up to P2_HOST_COPY_QB qubits keep a host copy of the state
- * (host_copy) after a second read, valid until the next change, so that long
- * runs of single-amplitude reads cost one download.
+ * (host_copy) after a read (from P2_GATHER_QB qubits on after a second one),
+ * valid until the next change, so that long runs of single-amplitude reads
+ * cost one download; a zeroed register is read without any.
  */
 #define P2_HOST_COPY_QB 16
+#define P2_GATHER_QB 13 /* FP32: 12 */
 
 struct p2_qreg {
 	struct p2_dev *dev;
@@ -52,7 +54,8 @@ struct p2_qreg {
 	double *wval;
 	size_t wlen, wcap;
 	double *host_copy;
-	enum { COPY_STALE = 0, COPY_VALID, COPY_READ_ONCE } host_copy_valid;
+	enum { COPY_STALE = 0, COPY_VALID, COPY_READ_ONCE,
+		COPY_ZERO } host_copy_valid;
 	struct p2_prog *rec; /* recording instead of executing, or NULL */
 	/* input of the plan held in passes/recs (a flush whose queue is
 	 * byte-identical, with the same settings, reuses it: every Trotter

@@ -377,9 +377,17 @@ int qreg_getamps(struct qreg *reg, const uint64_t *idx, _Complex double *z,
 	if (qreg_flush(reg) < 0)
 		return -1;
 	double *out = (double *)z; /* _Complex double = (re, im) */
+	if (b->host_copy && b->host_copy_valid == COPY_ZERO) {
+		memset(out, 0, sizeof(double) * 2 * n);
+		return 0;
+	}
 	/* the first read after a change gathers its few amplitudes; a second
-	 * one brings the whole state */
-	const int gather = n <= QREG_FEW && b->host_copy_valid == COPY_STALE;
+	 * one brings the whole state, as does the first of a narrow register,
+	 * where that costs little more (rotate and read once, us, gather /
+	 * state: FP64 8, 12, 13, 16 qubits 34 / 34, 35 / 39, 36 / 42, 35 / 98;
+	 * FP32 8, 11, 12 35 / 35, 35 / 40, 36 / 48) */
+	const int gather = n <= QREG_FEW && reg->qb_lo >= P2_GATHER_QB - (b->prec == PHASE2_PREC_FP32) &&
+		b->host_copy_valid == COPY_STALE;
 	if (b->host_copy && !gather) {
 		if (b->host_copy_valid != COPY_VALID) {
 			if (p2d_get_state(b->dev, b->host_copy) < 0) {
@@ -430,9 +438,11 @@ void qreg_zero(struct qreg *reg)
 			b->error = -1;
 		return;
 	}
-	b->host_copy_valid = COPY_STALE;
-	if (p2d_zero(b->dev) < 0)
+	b->host_copy_valid = COPY_ZERO;
+	if (p2d_zero(b->dev) < 0) {
 		b->error = -1;
+		b->host_copy_valid = COPY_STALE;
+	}
 }
 
 int qreg_get_state(struct qreg *reg, double *out)
@@ -442,6 +452,10 @@ int qreg_get_state(struct qreg *reg, double *out)
 		return -1;
 	if (b->host_copy && b->host_copy_valid == COPY_VALID) {
 		memcpy(out, b->host_copy, sizeof(double) * 2 * reg->namp);
+		return 0;
+	}
+	if (b->host_copy && b->host_copy_valid == COPY_ZERO) {
+		memset(out, 0, sizeof(double) * 2 * reg->namp);
 		return 0;
 	}
 	return p2d_get_state(b->dev, out);
