@@ -25,7 +25,7 @@
 template <int M>
 __device__ __forceinline__ void p2_batch_pass_tile(float2 *st,
 	const struct phase2_pass &p, uint64_t r0, uint64_t nrep, uint32_t cpt,
-	const struct p2_lift32_rec *srec, uint32_t lane)
+	const struct p2_lift32_short *srec, uint32_t lane)
 {
 	uint32_t pb[M > 0 ? M : 1];
 #pragma unroll
@@ -134,10 +134,10 @@ __device__ __forceinline__ void p2_batch_pass_tile64(double2 *st,
  * (FP64). */
 template <typename ST, bool X> struct p2_brec;
 template <> struct p2_brec<float2, false> {
-	typedef struct p2_lift32_rec type;
+	typedef struct p2_lift32_short type;
 	static __device__ __forceinline__ type of(const phase2_rot_rec &r)
 	{
-		return p2_lift32_of(r);
+		return p2_lift32_short_of(r);
 	}
 };
 template <> struct p2_brec<float2, true> {
@@ -267,6 +267,8 @@ __global__ void __launch_bounds__(P2_TPB,
 	typedef typename p2_brec<ST, X>::type RT;
 	/* each warp keeps the records of the pass it last ran */
 	__shared__ RT srec_all[P2_BATCH_WARPS][P2_MAX_ROTS_PER_PASS];
+	static_assert(p2_batch_blocks(F64, X) * (sizeof srec_all + 1024) <=
+			(228 << 10), "shared memory of the blocks of an SM");
 	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
 	RT *const srec = srec_all[wid];
 	const uint32_t nwarps = gridDim.x * P2_BATCH_WARPS;

@@ -809,6 +809,51 @@ __device__ __forceinline__ struct p2_lift32_rec p2_lift32_of(
 	return o;
 }
 
+/* The same in 24 bytes, the +-1 made when a rotation is applied: for the
+ * persistent kernel, each of whose warps holds the records of a whole pass
+ * (48 bytes a record would leave room for four blocks an SM, not five). */
+struct p2_lift32_short {
+	uint64_t z;
+	uint32_t key; /* W << 8 | U << 1 | odd */
+	uint32_t sm;
+	float t, s;
+};
+
+__device__ __forceinline__ struct p2_lift32_short p2_lift32_short_of(
+	const struct phase2_rot_rec &in)
+{
+	struct p2_lift32_short o;
+	o.z = in.z;
+	o.key = (uint32_t)in.W << 8 | ((uint32_t)in.U << 1) | in.odd;
+	o.sm = in.smask;
+	o.t = (float)in.c;
+	o.s = (float)in.s;
+	return o;
+}
+
+__device__ __forceinline__ const struct p2_lift32_rec &p2_lift32_full(
+	const struct p2_lift32_rec &q)
+{
+	return q;
+}
+
+__device__ __forceinline__ struct p2_lift32_rec p2_lift32_full(
+	const struct p2_lift32_short &q)
+{
+	struct p2_lift32_rec o;
+	o.z = q.z;
+	o.key = q.key & 0xffu;
+	o.sm = q.sm;
+	o.t = q.t;
+	o.s = q.s;
+#pragma unroll
+	for (int k = 0; k < PHASE2_MAX_SPAN; ++k)
+		o.m[k] = __uint_as_float(0x3f800000u |
+			(q.key << (23 - k) & 0x80000000u));
+	o.pad = 0.f;
+	return o;
+}
+
 /*
  * One coset of a lifted FP32 pass: load the 2^M amplitudes x ^ off(u)
  * into FP32 registers, apply the run of rotations, store them (negated
@@ -816,10 +861,10 @@ __device__ __forceinline__ struct p2_lift32_rec p2_lift32_of(
  * persistent batch kernel, whose blocks read what other blocks of the same
  * launch wrote).
  */
-template <int M, typename IT, bool CG, bool PK>
+template <int M, typename IT, bool CG, bool PK, typename RT>
 __device__ __forceinline__ void p2_lift32_coset(float2 *__restrict__ st, IT x,
-	const IT (&pb)[M > 0 ? M : 1], const struct p2_lift32_rec *srec,
-	uint32_t nrot, uint32_t negm)
+	const IT (&pb)[M > 0 ? M : 1], const RT *srec, uint32_t nrot,
+	uint32_t negm)
 {
 	float re[1 << M], im[1 << M];
 #pragma unroll
@@ -834,7 +879,7 @@ __device__ __forceinline__ void p2_lift32_coset(float2 *__restrict__ st, IT x,
 		im[u] = v.y;
 	}
 	for (uint32_t r = 0; r < nrot; ++r) {
-		const struct p2_lift32_rec q = srec[r];
+		const struct p2_lift32_rec q = p2_lift32_full(srec[r]);
 		p2_apply_lift32<M, PK>(q, re, im, p2_parity(x & (IT)q.z));
 	}
 	const IT xs = p2_opaque(x);
