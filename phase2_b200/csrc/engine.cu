@@ -1668,7 +1668,8 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 		return 0;
 	const int form = passes[0].form;
 	const bool split = p2_split_ok(d, form);
-	const bool tile = p2_tile_ok(d, form, npass, nrec);
+	const bool tile = p2_tile_ok(d, form, passes, npass, recs,
+		nrec);
 	const bool resident = split || tile || p2_resident_ok(d, form);
 	struct p2_graph *g = resident
 		? NULL

@@ -319,7 +319,9 @@ cudaError_t p2_resident_progs(const struct p2_dev *d, uint32_t nqb, uint32_t g,
 /* tile.cu: FP64 registers beyond the caches: whether a flush's rotations run
  * regrouped into tile runs, and their launches, as p2_resident_run; *trips:
  * state round trips. */
-bool p2_tile_ok(const struct p2_dev *d, int form, size_t npass, size_t nrec);
+bool p2_tile_ok(const struct p2_dev *d, int form,
+	const struct phase2_pass *passes, size_t npass,
+	const struct phase2_rot_rec *recs, size_t nrec);
 int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
 	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
 	uint64_t plan_id, size_t *trips);

@@ -215,11 +215,39 @@ __global__ void __launch_bounds__(P2_TILE_TPB, 2) k_tile(
  * (1.96) / 1.89 (1.97), 250 a pass 1.88 (1.90) / 2.22 (2.16) / 2.27 (2.17)
  * / 2.28 (2.17).  Runs of 128 bytes (9 dimensions beside 3 low qubits, 9.9
  * draws a trip) gave 0.86 / 1.15 / 1.16 / 1.14.
+ *
+ * A short flush whose runs are as many as its passes gains nothing by them
+ * (us, pass kernels / tiles: 10 random strings, two passes, at 22, 24, 28
+ * qubits 53 / 56, 183 / 209, 2849 / 3337; 5 strings 28 / 34, 95 / 102, 1367
+ * / 1409), except one of few rotations with one mask, which a pass reads in
+ * short runs (1 and 4 of them at 22 qubits 29 / 22, 29 / 26, at 24 97 / 95,
+ * 98 / 98, at 28 1428 / 1426, 1439 / 1457), and one pass again at 20 qubits,
+ * where the launch bounds it (16 / 10).  Long ones always gain.
  */
-bool p2_tile_ok(const struct p2_dev *d, int form, size_t npass, size_t nrec)
+static bool short_gain(const struct phase2_pass *passes, size_t npass,
+	const struct phase2_rot_rec *recs, size_t nrec)
+{
+	if (npass > 4 || p2_tile_count(passes, npass, recs) < npass)
+		return true;
+	if (npass > 1 || nrec > 6)
+		return false;
+	uint32_t mask = 0;
+	for (size_t i = 0; i < nrec; i++) {
+		if (mask && recs[i].U && recs[i].U != mask)
+			return false;
+		mask |= recs[i].U;
+	}
+	return true;
+}
+
+bool p2_tile_ok(const struct p2_dev *d, int form,
+	const struct phase2_pass *passes, size_t npass,
+	const struct phase2_rot_rec *recs, size_t nrec)
 {
 	return form == PHASE2_FORM_EXACT && d->tiles &&
-		d->nqb >= P2_TILE_MIN_QB && nrec <= 10 * npass;
+		d->nqb >= P2_TILE_MIN_QB && nrec <= 10 * npass &&
+		((npass == 1 && d->nqb == P2_TILE_MIN_QB) ||
+			short_gain(passes, npass, recs, nrec));
 }
 
 int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,

@@ -155,6 +155,50 @@ static inline uint32_t p2_tile_subs(struct p2_tile *t, const uint32_t *fl,
 	return n;
 }
 
+/* An empty run's echelon: the low qubits, which are in every tile. */
+static inline void p2_tile_open(struct p2_tile_ech *e)
+{
+	memset(e, 0, sizeof *e);
+	for (int q = 0; q < P2_TILE_LOW; q++)
+		p2_te_add(e, UINT64_C(1) << q);
+}
+
+/* Add flip mask f to a run of n rotations: 0 if it is full. */
+static inline int p2_tile_take(struct p2_tile_ech *e, uint32_t n, uint64_t f)
+{
+	if (n == P2_TILE_ROTS)
+		return 0;
+	const uint64_t v = p2_te_reduce(e, f);
+	if (v) {
+		if (e->rows == P2_TILE_BITS)
+			return 0;
+		p2_te_add(e, v);
+	}
+	return 1;
+}
+
+/* The runs that p2_tile_build makes of these passes. */
+static inline size_t p2_tile_count(const struct phase2_pass *passes,
+	size_t npass, const struct phase2_rot_rec *recs)
+{
+	struct p2_tile_ech e;
+	size_t runs = 0;
+	uint32_t n = 0;
+	for (size_t p = 0; p < npass; p++)
+		for (uint32_t r = 0; r < passes[p].nrot; r++) {
+			const uint64_t f = p2_rec_flip(&passes[p],
+				&recs[passes[p].rot_off + r]);
+			if (runs == 0 || !p2_tile_take(&e, n, f)) {
+				p2_tile_open(&e);
+				p2_tile_take(&e, 0, f);
+				runs++;
+				n = 0;
+			}
+			n++;
+		}
+	return runs;
+}
+
 /*
  * The flush's rotations in order, greedily: a tile run takes rotations while
  * their flips span at most P2_TILE_BITS - P2_TILE_LOW dimensions beside the
@@ -174,21 +218,15 @@ static inline uint32_t p2_tile_build(const struct phase2_pass *passes,
 		uint64_t flip[P2_TILE_ROTS];
 		uint32_t fl[P2_TILE_ROTS];
 		memset(t, 0, sizeof *t);
-		memset(&e, 0, sizeof e);
-		for (int q = 0; q < P2_TILE_LOW; q++)
-			p2_te_add(&e, UINT64_C(1) << q);
+		p2_tile_open(&e);
 		t->rot_off = (uint32_t)i;
 		t->sub_off = ns;
-		for (; i < nrec && t->nrot < P2_TILE_ROTS; i++) {
+		for (; i < nrec; i++) {
 			while (p + 1 < npass && i >= passes[p + 1].rot_off)
 				p++;
 			const uint64_t f = p2_rec_flip(&passes[p], &recs[i]);
-			const uint64_t v = p2_te_reduce(&e, f);
-			if (v) {
-				if (e.rows == P2_TILE_BITS)
-					break;
-				p2_te_add(&e, v);
-			}
+			if (!p2_tile_take(&e, t->nrot, f))
+				break;
 			flip[t->nrot++] = f;
 		}
 		for (int q = 0; e.rows < P2_TILE_BITS; q++) {
