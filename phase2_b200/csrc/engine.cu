@@ -1660,6 +1660,24 @@ static struct p2_graph *graph_for(struct p2_dev *d,
 	return NULL;
 }
 
+/*
+ * A flush that the pass kernels end sooner unless it is the last one again,
+ * whose plan is on the device: one pass, where cutting it costs the
+ * host as much as the kernel gains and the cluster launch and barriers
+ * outlast it (rotate and wait, us, pass kernel / resident or split: one
+ * string at 8, 12, 14, 17 qubits 21.0 / 22.1, 21.4 / 23.8, 21.5 / 24.6,
+ * 21.6 / 22.9; 16 strings of two masks 24.6 / 27.1 at 11, 28.8 / 30.6 at
+ * 19; queued without waiting, 32 strings 16.8 / 20.3 at 12, 18.6 / 24.1 at
+ * 19).  Up to 10 qubits longer passes are better cut (20 random strings of
+ * 5 qubits, FP32, 19.5 / 16.3).  At 14 qubits two passes too, which a graph
+ * replays (repeated 12.9 / 14.9, rotate and wait 24.2 / 28.3).
+ */
+static bool brief_flush(const struct p2_dev *d, size_t npass, size_t nrec)
+{
+	return npass == 1 && nrec <= (d->nqb <= 10 ? 8 : 64) &&
+		d->nqb <= 20;
+}
+
 extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
 	uint64_t plan_id)
@@ -1667,10 +1685,15 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	if (npass == 0)
 		return 0;
 	const int form = passes[0].form;
-	const bool split = p2_split_ok(d, form);
-	const bool tile = p2_tile_ok(d, form, passes, npass, recs,
+	const bool again = plan_id != 0 && plan_id == d->last_plan;
+	d->last_plan = plan_id;
+	const bool brief = !again && brief_flush(d, npass, nrec);
+	const bool split = !brief && p2_split_ok(d, form);
+	const bool tile = !brief && p2_tile_ok(d, form, passes, npass, recs,
 		nrec);
-	const bool resident = split || tile || p2_resident_ok(d, form);
+	const bool resident = split || tile ||
+		(!brief && !(d->nqb == 14 && npass == 2) &&
+			p2_resident_ok(d, form));
 	struct p2_graph *g = resident
 		? NULL
 		: graph_for(d, passes, npass, recs, nrec);

@@ -59,6 +59,7 @@ struct p2_dev {
 	cudaStream_t stream;
 	int sm_count;
 	int tiles;        /* passes may be regrouped (p2d_set_tiles) */
+	uint64_t last_plan; /* number of the last flush's plan */
 	int device;       /* of the shell (engine.cu) */
 	uint64_t context;
 

@@ -49,3 +49,33 @@ def test_wide_exact(n, count, one_mask, replays):
     want, _ = _run(n, p2.PREC_FP64, (1, 1), [a, a])
     assert np.array_equal(got, want)
     assert st["graph_replays"] == replays
+
+
+@pytest.mark.parametrize("count", [1, 5, 8])
+@pytest.mark.parametrize("n", [3, 5, 10, 11, 13, 14, 15, 19, 20])
+def test_narrow(n, count):
+    a = _flush(n, count, True, count)
+    b = _flush(n, count, True, count + 100)
+    # two flushes in turn: pass kernels; the same again: its plan is kept
+    turns = [a, b, a, b]
+    got, st = _run(n, p2.PREC_FP64, (5, 0), turns)
+    assert st["graph_replays"] == 0
+    assert np.array_equal(got, _run(n, p2.PREC_FP64, (1, 1), turns)[0])
+    again = [a, a, a, b, a]
+    got, st = _run(n, p2.PREC_FP64, (5, 0), again)
+    assert st["graph_replays"] == 1
+    assert np.array_equal(got, _run(n, p2.PREC_FP64, (1, 1), again)[0])
+
+
+@pytest.mark.parametrize("count", [1, 5, 8, 10])
+@pytest.mark.parametrize("n", [5, 11, 14, 17])
+def test_fp32_routes_agree(n, count):
+    """The second of two equal flushes runs as sub-passes: the bits of the
+    pass kernels, which run it on another register."""
+    a = _flush(n, count, count < 10, 7 * count)
+    first = _run(n, p2.PREC_FP32, (5, 0), [a])[0]
+    got = _run(n, p2.PREC_FP32, (5, 0), [a, a])[0]
+    with Register(n, p2.PREC_FP32) as r:
+        r.set_state(first)
+        r.paulirot(*a)
+        assert np.array_equal(r.get_state(), got)
