@@ -692,6 +692,55 @@ static void batch_account(struct p2_dev *const *devs,
 	d0->h2d_bytes += tables;
 }
 
+/* As many programs of the largest one's work as the batch's work makes. */
+static uint32_t batch_even(struct p2_dev *const *devs,
+	const struct p2_prog *const *progs, size_t n)
+{
+	double work = 1.0, most = 1.0;
+	for (size_t i = 0; i < n; i++) {
+		const double w = (double)progs[i]->rotations * devs[i]->namp;
+		work += w;
+		if (w > most)
+			most = w;
+	}
+	return (uint32_t)(work / most + 0.999);
+}
+
+/*
+ * Whether a batch whose registers all fit on chip runs there.  A 14-qubit
+ * program takes two SMs, and once those have to wait for one another the
+ * persistent kernel, which shares every SM among programs, is faster: FP32
+ * from half as many programs as SMs on, FP64 from twice that with few
+ * rotations a pass (kernel us, on chip / persistent: FP32 trott 64, 100,
+ * 148, 300 programs 277 / 319, 498 / 402, 532 / 562, 1152 / 914, draws 609 /
+ * 921, 1008 / 1041, 1167 / 1114, 2324 / 1490; FP64 trott 148, 300 556 / 612,
+ * 1231 / 1318, draws 1152 / 1148, 2251 / 1905).
+ */
+static bool batch_fits(struct p2_dev *const *devs,
+	const struct p2_prog *const *progs, size_t n)
+{
+	uint64_t rots = 0, passes = 0;
+	uint32_t nqb = 0;
+	for (size_t i = 0; i < n; i++) {
+		if (!p2_resident_prog_ok(devs[i], progs[i]->npass
+				    ? progs[i]->passes[0].form
+				    : PHASE2_FORM_EXACT))
+			return false;
+		if (devs[i]->nqb > nqb)
+			nqb = devs[i]->nqb;
+		for (size_t k = 0; k < progs[i]->npass; k++)
+			rots += progs[i]->passes[k].nrot;
+		passes += progs[i]->npass;
+	}
+	if (nqb < 14)
+		return true;
+	const uint32_t even = batch_even(devs, progs, n);
+	const uint32_t sms = (uint32_t)devs[0]->sm_count;
+	return devs[0]->prec == PHASE2_PREC_FP64
+		? even <= sms || rots >= 10 * passes
+		: 2 * even <= sms;
+}
+
 /*
  * A batch whose registers all fit on chip: every program's passes cut into
  * sub-passes, its ops into runs of them, and one launch of k_resident_prog.
@@ -707,12 +756,7 @@ static int batch_on_chip(struct p2_dev *const *devs,
 	struct p2_dev *d0 = devs[0];
 	size_t nops = 0, nrec = 0, nw = 0, ng = 0;
 	uint32_t nqb = 0;
-	double work = 1.0, most = 1.0;
 	for (size_t i = 0; i < n; i++) {
-		const double w = (double)progs[i]->rotations * devs[i]->namp;
-		work += w;
-		if (w > most)
-			most = w;
 		nops += progs[i]->nops;
 		nrec += progs[i]->nrec;
 		nw += progs[i]->nw;
@@ -837,7 +881,7 @@ static int batch_on_chip(struct p2_dev *const *devs,
 		 * whose work is that of four: 4.5 ms on 4 blocks each, 2.4 on
 		 * 16) */
 		e = p2_resident_progs(d0, nqb, (uint32_t)n,
-			(uint32_t)(work / most + 0.999),
+			batch_even(devs, progs, n),
 			(const struct p2_res_prog *)b,
 			(const uint64_t *)(b + o_widx),
 			(const double *)(b + o_wval),
@@ -891,12 +935,7 @@ extern "C" int p2d_batch_run(struct p2_dev *const *devs,
 		log_error("batch: program too large");
 		return -1;
 	}
-	bool on_chip = true;
-	for (size_t i = 0; i < n && on_chip; i++)
-		on_chip = p2_resident_prog_ok(devs[i], progs[i]->npass
-				? progs[i]->passes[0].form
-				: PHASE2_FORM_EXACT);
-	if (on_chip)
+	if (batch_fits(devs, progs, n))
 		return batch_on_chip(devs, progs, n, gout, kernel_ms);
 	/* one device buffer: uploaded part, then outputs and control */
 	const size_t o_inst = 0;

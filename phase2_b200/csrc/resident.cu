@@ -712,7 +712,11 @@ cudaError_t p2_resident_progs(const struct p2_dev *d, uint32_t nqb, uint32_t g,
 	const double *wval, const uint64_t *gidx, double2 *gout,
 	struct p2_bctl *ctl, unsigned long long *start)
 {
-	const uint32_t lb = res_sample_blocks(nqb, d->sm_count, even);
+	uint32_t lb = res_sample_blocks(nqb, d->sm_count, even);
+	/* at 14 qubits a program has two blocks in any case: four each, as
+	 * long as an SM in eight stays free for the clusters to fit in */
+	if (nqb == 14 && lb == 1 && (even << 2) <= (uint32_t)d->sm_count * 7 / 8)
+		lb = 2;
 	return d->prec == PHASE2_PREC_FP64
 		? res_launch_progs<double2, false>(nqb, lb, g, d->stream, progs,
 			  widx, wval, gidx, gout, ctl, start)
