@@ -766,7 +766,18 @@ static int io_reserve(struct p2_dev *d, size_t n)
  * nothing until the next one is created.
  */
 #define P2_SHELLS 32
-#define P2_SHELL_BYTES ((size_t)2 << 20)
+#define P2_SHELL_BYTES ((size_t)3 << 20)
+
+/* Two staging buffers grown by full flushes (a record, and its copy with a
+ * sub-pass of twice its size, in a power of two) and a flush's device
+ * records, with a quarter left for the small buffers: one that flushed more
+ * than 5461 rotations at a time would else be given up. */
+#define P2_STAGE_MAX (32768 * sizeof(struct phase2_rot_rec))
+static_assert(3 * P2_QUEUE_FLUSH <= 32768 &&
+		2 * P2_STAGE_MAX +
+				P2_QUEUE_FLUSH * sizeof(struct phase2_rot_rec) <=
+			P2_SHELL_BYTES / 4 * 3,
+	"a register with full flushes is kept");
 
 static pthread_mutex_t shell_lock = PTHREAD_MUTEX_INITIALIZER;
 static struct p2_dev *shells[P2_SHELLS];
