@@ -55,7 +55,8 @@ FORM_LIFTED, FORM_LIFTED_F32 = 1, 2
 def _probe_rotations(nqb: int, M: int, groups: int, seed: int):
     """`groups` runs of M rotations with independent random flips (2-4
     qubits each) plus one diagonal term: each run plans to one pass of
-    span M."""
+    span M under the limit of M + 1 rotations a pass (which also keeps the
+    passes from being regrouped into tile runs)."""
     rng = np.random.Generator(np.random.PCG64(seed))
     flip, phase = [], []
     for _ in range(groups):
@@ -90,7 +91,7 @@ def sweep_launch(nqb: int, groups: int = 12, reps: int = 2) -> dict:
         elem = 16 if prec == PREC_FP64 else 8
         with Register(nqb, prec) as reg:
             for M in range(1, 6):
-                reg.set_fusion(M, 0)
+                reg.set_fusion(M, M + 1)
                 flip, phase, phi = _probe_rotations(nqb, M, groups, 7 + M)
                 best = None
                 trials = []
@@ -274,7 +275,7 @@ def probe(nqb: int, pname: str, M: int, variant: int, per_sm: int,
     flip, phase, phi = _probe_rotations(nqb, M, groups, 7 + M)
     elem = 16 if prec == PREC_FP64 else 8
     with Register(nqb, prec) as reg:
-        reg.set_fusion(M, 0)
+        reg.set_fusion(M, M + 1)
         _time_passes(reg, flip[:M + 1], phase[:M + 1], phi[:M + 1])
         ms, passes = _time_passes(reg, flip, phase, phi)
     return {"prec": pname, "M": M, "variant": variant, "per_sm": per_sm,
