@@ -473,9 +473,8 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 	const uint32_t C = (uint32_t)((T + P2_QUEUE_FLUSH - 1) / P2_QUEUE_FLUSH);
 	/* registers that fit on chip: no state copies, no persistent kernel */
 	const bool whole = T > 0 && p2_onchip_samples_ok(d, job->form, G);
-	const bool subs = T > 0 && !whole &&
-		p2_resident_samples_ok(d, job->form);
-	const bool res = whole || subs;
+	bool subs = T > 0 && !whole && p2_resident_samples_ok(d, job->form);
+	bool res = whole || subs;
 	if (res) {
 		R = 1;
 		/* twice the scratch a rotation */
@@ -538,6 +537,9 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 			R = 1;
 		} else if (G > 1) {
 			G = (G + 1) / 2;
+		} else if (subs) {
+			/* the persistent kernel needs no sub-passes */
+			subs = res = false;
 		} else {
 			log_error("device sampling: no room for %zu bytes of "
 				  "scratch", total);

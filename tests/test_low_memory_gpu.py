@@ -1,0 +1,52 @@
+"""Little free device memory, in a child process that holds the rest: device
+sampling falls back on the kernel that needs less scratch, with the same
+bits."""
+
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import numpy as np, torch
+import phase2_b200 as p2
+from phase2_b200 import Register, workloads
+
+def leave(mib):
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty(free - (mib << 20), dtype=torch.uint8, device="cuda")
+
+p2.world_ensure()
+with Register(20, p2.PREC_FP64) as r:
+    r.norm2()
+"""
+
+SAMPLING = """
+t = workloads.jw_terms(8, 60, seed=1)
+d = workloads.hamming_dets(8, 1, 4, seed=2)
+def run():
+    return p2.qdrift(8, t, d, 3, 1 << 21, 1e-4, 7, with_stats=True,
+                     with_state=True)
+held = leave(480)
+a, sa = run()
+del held
+torch.cuda.empty_cache()
+b, sb = run()
+assert np.array_equal(a, b) and np.array_equal(sa["state"], sb["state"])
+print("done")
+"""
+
+
+def _child(code):
+    r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT,
+                       timeout=600, capture_output=True, text=True)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
+def test_device_sampling_without_room_for_sub_passes():
+    _child(SAMPLING)
