@@ -519,6 +519,7 @@ extern "C" int phase2_batch_wait_check(unsigned int idle_limit)
 	cudaFree(buf);
 	if (e != cudaSuccess) {
 		log_error("batch wait check: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 		return -1;
 	}
 	return status ? 1 : 0;
@@ -903,6 +904,7 @@ static int batch_on_chip(struct p2_dev *const *devs,
 	p2_scratch_free(b, d0->stream);
 	if (e != cudaSuccess) {
 		log_error("batch: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 		return -1;
 	}
 	if (kernel_ms)
@@ -971,6 +973,7 @@ extern "C" int p2d_batch_run(struct p2_dev *const *devs,
 		p2_batch_kernel(kind), P2_TPB, 0);
 	if (e != cudaSuccess) {
 		log_error("batch: setup: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 		return -1;
 	}
 	unsigned grid =
@@ -1075,6 +1078,7 @@ extern "C" int p2d_batch_run(struct p2_dev *const *devs,
 	if (e != cudaSuccess) {
 		p2_scratch_free(dbuf, d0->stream);
 		log_error("batch: setup: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 		return -1;
 	}
 	cudaEventRecord(d0->t0, d0->stream);
@@ -1114,6 +1118,7 @@ extern "C" int p2d_batch_run(struct p2_dev *const *devs,
 			p2_now() - tb4);
 	if (e != cudaSuccess) {
 		log_error("batch: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 		return -1;
 	}
 	if (status) {

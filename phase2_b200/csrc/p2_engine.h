@@ -109,6 +109,7 @@ struct p2_dev {
 		cudaError_t e_ = (call);                                       \
 		if (e_ != cudaSuccess) {                                       \
 			log_error("%s: %s", (what), cudaGetErrorString(e_));  \
+			cudaGetLastError(); /* reported here only */           \
 			return -1;                                             \
 		}                                                              \
 	} while (0)

@@ -796,6 +796,7 @@ extern "C" int p2d_sampled_device(struct p2_dev *d,
 		rc = 0;
 	} else {
 		log_error("device sampling: %s", cudaGetErrorString(e));
+		cudaGetLastError();
 	}
 	free(gidx);
 	free(hinst);

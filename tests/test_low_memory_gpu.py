@@ -1,6 +1,6 @@
 """Little free device memory, in a child process that holds the rest: device
 sampling falls back on the kernel that needs less scratch, with the same
-bits."""
+bits, and a call that fails leaves other registers alone."""
 
 import subprocess
 import sys
@@ -41,6 +41,19 @@ assert np.array_equal(a, b) and np.array_equal(sa["state"], sb["state"])
 print("done")
 """
 
+FAILURE = """
+held = leave(480)
+with Register(17, p2.PREC_FP64) as a, Register(12, p2.PREC_FP64) as b:
+    try:
+        a.getamps(np.zeros(1 << 25, dtype=np.uint64))
+    except RuntimeError:
+        b.setamps([5], [2.0])
+        b.paulirot(np.array([5], dtype=np.uint64),
+                   np.array([0], dtype=np.uint64), np.array([0.0]))
+        assert b.norm2() == 4.0
+        print("done")
+"""
+
 
 def _child(code):
     r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT,
@@ -50,3 +63,7 @@ def _child(code):
 
 def test_device_sampling_without_room_for_sub_passes():
     _child(SAMPLING)
+
+
+def test_failure_stays_with_its_register():
+    _child(FAILURE)
