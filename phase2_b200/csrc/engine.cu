@@ -918,10 +918,10 @@ static void pool_trim(void)
 static void shell_give(struct p2_dev *d)
 {
 	bool closed = false;
-	/* a register whose stream reports an error, or whose status word was
-	 * never read, is not reused */
+	/* a register whose stream reports an error, whose status word was
+	 * never read, or whose buffers could not all be had, is not reused */
 	bool keep = cudaStreamSynchronize(d->stream) == cudaSuccess &&
-		!d->status_pending;
+		!d->status_pending && (d->io_cap || !d->d_idx);
 	const size_t held = (d->d_recs_cap + d->h_recs_cap[0] +
 				    d->h_recs_cap[1]) *
 			sizeof(struct phase2_rot_rec) +

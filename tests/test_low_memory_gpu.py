@@ -54,6 +54,19 @@ with Register(17, p2.PREC_FP64) as a, Register(12, p2.PREC_FP64) as b:
         print("done")
 """
 
+LEAK = """
+held = leave(480)
+a = Register(17, p2.PREC_FP64)
+a.norm2()
+before = torch.cuda.mem_get_info()[0]
+try:
+    a.getamps(np.zeros(1 << 25, dtype=np.uint64))
+except RuntimeError:
+    a.close()
+    assert torch.cuda.mem_get_info()[0] > before - (32 << 20)
+    print("done")
+"""
+
 
 def _child(code):
     r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT,
@@ -63,6 +76,10 @@ def _child(code):
 
 def test_device_sampling_without_room_for_sub_passes():
     _child(SAMPLING)
+
+
+def test_failed_register_keeps_nothing():
+    _child(LEAK)
 
 
 def test_failure_stays_with_its_register():
