@@ -720,7 +720,7 @@ static uint32_t batch_even(struct p2_dev *const *devs,
 static bool batch_fits(struct p2_dev *const *devs,
 	const struct p2_prog *const *progs, size_t n)
 {
-	uint64_t rots = 0, passes = 0;
+	size_t rots = 0, passes = 0;
 	uint32_t nqb = 0;
 	for (size_t i = 0; i < n; i++) {
 		if (!p2_resident_prog_ok(devs[i], progs[i]->npass
@@ -729,8 +729,7 @@ static bool batch_fits(struct p2_dev *const *devs,
 			return false;
 		if (devs[i]->nqb > nqb)
 			nqb = devs[i]->nqb;
-		for (size_t k = 0; k < progs[i]->npass; k++)
-			rots += progs[i]->passes[k].nrot;
+		rots += progs[i]->nrec;
 		passes += progs[i]->npass;
 	}
 	if (nqb < 14)
