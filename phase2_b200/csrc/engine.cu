@@ -508,6 +508,20 @@ __global__ void k_gather_few(const ST *__restrict__ st,
 	}
 }
 
+/* A small state to pinned host memory, as doubles.  A copy queued behind a
+ * kernel starts 8 us after its end, the next kernel 1 us. */
+template <typename ST>
+__global__ void k_state_out(const ST *__restrict__ st, uint32_t n,
+	double2 *__restrict__ out)
+{
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i < n) {
+		double re, im;
+		p2_ld(st, i, re, im);
+		out[i] = make_double2(re, im);
+	}
+}
+
 /* Neumaier: s + c carries the running sum and its rounding error. */
 __device__ __forceinline__ void p2_neumaier(double &s, double &c, double v)
 {
@@ -1215,12 +1229,15 @@ extern "C" int p2d_get(struct p2_dev *d, const uint64_t *idx, double *z,
 }
 
 /*
- * Small states are read through the pinned staging: a pageable copy costs a
- * few microseconds more to start, 15 more at 1 MiB.  FP32 ones are also
- * widened, and reading what was just written by the device is slow there
- * (rotate and read, us, 12 / 14 / 16 qubits, staged / not: FP64 37 / 49 / 94,
- * 41 / 55 / 109; FP32 47 / 87 / 251, 49 / 71 / 170).
+ * Small states are read through the pinned staging, the smallest by a kernel:
+ * a pageable copy costs a few microseconds more to start, 15 more at 1 MiB.
+ * FP32 ones are also widened, and reading what was just written by the device
+ * is slow on the host (rotate, wait and read, us, 14 / 16 qubits, staged /
+ * not: FP64 49 / 94, 55 / 109; FP32 87 / 251, 71 / 170; by the kernel at 12
+ * FP64 36, 41 pageable, FP32 41, 49).
  */
+#define P2_READ_KERNEL (UINT64_C(1) << 12)
+
 static bool read_staged(const struct p2_dev *d)
 {
 	return d->namp <= (UINT64_C(1) << 16) &&
@@ -1232,6 +1249,25 @@ extern "C" int p2d_get_state(struct p2_dev *d, double *out)
 	const size_t bytes = d->namp * sizeof(double2);
 	if (p2_status_check(d) < 0)
 		return -1;
+	if (d->namp <= P2_READ_KERNEL) {
+		void *const h = p2_stage_reserve(d, (bytes + 31) / 32);
+		if (!h)
+			return -1;
+		const uint32_t n = (uint32_t)d->namp;
+		const unsigned grid = (n + 127) / 128;
+		if (d->prec == PHASE2_PREC_FP64)
+			k_state_out<<<grid, 128, 0, d->stream>>>(
+				(const double2 *)d->state, n, (double2 *)h);
+		else
+			k_state_out<<<grid, 128, 0, d->stream>>>(
+				(const float2 *)d->state, n, (double2 *)h);
+		d->launches++;
+		d->d2h_bytes += bytes;
+		CUDA_OK(cudaGetLastError(), "state read launch");
+		CUDA_OK(cudaStreamSynchronize(d->stream), "state read");
+		memcpy(out, h, bytes);
+		return 0;
+	}
 	if (read_staged(d)) {
 		void *const h = p2_stage_reserve(d, (d->namp * d->elem + 31) / 32);
 		if (!h)

@@ -38,7 +38,7 @@ void p2_settings_from_env(void);
  * cost one download; a zeroed register is read without any.
  */
 #define P2_HOST_COPY_QB 16
-#define P2_GATHER_QB 13 /* FP32: 12 */
+#define P2_GATHER_QB 10
 
 struct p2_qreg {
 	struct p2_dev *dev;

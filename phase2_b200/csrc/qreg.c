@@ -383,10 +383,10 @@ int qreg_getamps(struct qreg *reg, const uint64_t *idx, _Complex double *z,
 	}
 	/* the first read after a change gathers its few amplitudes; a second
 	 * one brings the whole state, as does the first of a narrow register,
-	 * where that costs little more (rotate and read once, us, gather /
-	 * state: FP64 8, 12, 13, 16 qubits 34 / 34, 35 / 39, 36 / 42, 35 / 98;
-	 * FP32 8, 11, 12 35 / 35, 35 / 40, 36 / 48) */
-	const int gather = n <= QREG_FEW && reg->qb_lo >= P2_GATHER_QB - (b->prec == PHASE2_PREC_FP32) &&
+	 * where that costs no more (rotate and read once, us, gather / state,
+	 * FP64: 8 qubits 27 / 28, 10 28 / 30, 11 28 / 33, 16 28 / 104; twice
+	 * 45 / 35 at 8 and 50 / 35 at 10, but drivers read a step once) */
+	const int gather = n <= QREG_FEW && reg->qb_lo >= P2_GATHER_QB &&
 		b->host_copy_valid == COPY_STALE;
 	if (b->host_copy && !gather) {
 		if (b->host_copy_valid != COPY_VALID) {

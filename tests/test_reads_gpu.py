@@ -16,7 +16,7 @@ def _world():
 
 
 @pytest.mark.parametrize("prec", [p2.PREC_FP64, p2.PREC_FP32])
-@pytest.mark.parametrize("n", [1, 8, 12, 13, 14, 16])
+@pytest.mark.parametrize("n", [1, 9, 10, 12, 13, 16])
 def test_copies_and_values(n, prec):
     rng = np.random.Generator(np.random.PCG64(n))
     amp = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
@@ -32,7 +32,7 @@ def test_copies_and_values(n, prec):
         assert r.getamps([last])[0] == amp[last]
         first = copies(r)
         assert np.array_equal(r.getamps([0, last]), amp[[0, last]])
-        if n < 12:
+        if n < 10:
             assert copies(r) == first
         second = copies(r)
         assert np.array_equal(r.get_state(), amp)
