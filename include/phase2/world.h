@@ -43,7 +43,10 @@ struct world_info {
  * Returns WORLD_READY or WORLD_ERR (reference: world.h:54). */
 int world_init(int *argc, char ***argv, uint64_t seed);
 
-/* Returns WORLD_DONE or WORLD_ERR (reference: world.h:66). */
+/* Also gives back what destroyed registers left for later ones: device
+ * memory in the default pool (up to a sixteenth of the device's), streams and
+ * staging.  Registers still there keep working and leave nothing.
+ * Returns WORLD_DONE or WORLD_ERR (reference: world.h:66). */
 int world_free(void);
 
 /* Snapshot of the world state; returns wd->stat (reference: world.h:75). */

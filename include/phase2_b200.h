@@ -331,7 +331,8 @@ struct phase2_stats {
 	uint64_t d2h_bytes; /* device-to-host bytes copied for this register */
 	uint64_t graph_replays; /* flushes launched from a plan kept on the
 				 * device (seen before, e.g. every Trotter
-				 * step after the first or second): a captured
+				 * step after the first or second; a flush of
+				 * one pass after the second): a captured
 				 * CUDA graph (registers of up to 24 qubits),
 				 * or kept sub-passes and tile runs */
 	uint64_t sweeps;    /* state round trips as planned: one per pass, one

@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(P2_TPB, p2_min_blocks(M))
  * from HBM (2^M independent 8-byte loads, coalesced across the warp),
  * widens to FP64, applies the run of rotations in registers and narrows
  * once at the store.  Index arithmetic is 32-bit when IT is uint32_t.
- * At M = 5, three resident blocks cap a thread at 168 registers (a few
- * spilled); measured faster than two blocks with no spills.
+ * At M = 5, three resident blocks cap a thread at 168 registers (160 used,
+ * no spills); measured faster than two blocks.
  */
 template <int M, typename IT>
 __global__ void __launch_bounds__(P2_TPB, M >= 5 ? 3 : p2_min_blocks(M))
