@@ -2083,14 +2083,9 @@ void p2_scratch_free(void *p, cudaStream_t stream)
 #define P2_NOALLOC_MAX_BLOCKS 8192
 #define P2_NOALLOC_CHUNK (UINT64_C(1) << 21)
 #define P2_NOALLOC_MAX_AMPS ((uint64_t)P2_NOALLOC_MAX_BLOCKS * P2_NOALLOC_CHUNK)
-#define P2_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) double
 	p2_noalloc_scratch[2 * P2_NOALLOC_MAX_BLOCKS];
-
-/* Address of the array on each device, looked up by the first call there
- * (written once with the same value by any thread that races on it). */
-static double *p2_noalloc_addr[P2_NOALLOC_MAX_DEVICES];
 
 extern "C" int phase2_norm2_noalloc(const void *d_state, int prec,
 	uint64_t namp, double *d_out, void *stream)
@@ -2131,18 +2126,11 @@ extern "C" int phase2_norm2_noalloc(const void *d_state, int prec,
 		return -1;
 	int dev = 0;
 	CUDA_OK(cudaGetDevice(&dev), "phase2_norm2_noalloc: current device");
-	if (dev < 0 || dev >= P2_NOALLOC_MAX_DEVICES) {
-		log_error("phase2_norm2_noalloc: device %d beyond the %d"
-			  " supported", dev, P2_NOALLOC_MAX_DEVICES);
-		return -1;
-	}
-	double *part = __atomic_load_n(&p2_noalloc_addr[dev], __ATOMIC_ACQUIRE);
-	if (!part) {
-		/* first call on this device: resolve the array's address */
-		CUDA_OK(cudaGetSymbolAddress((void **)&part, p2_noalloc_scratch),
-			"phase2_norm2_noalloc: scratch address");
-		__atomic_store_n(&p2_noalloc_addr[dev], part, __ATOMIC_RELEASE);
-	}
+	/* looked up by every call (no allocation, no wait): a device reset
+	 * moves the array */
+	double *part = NULL;
+	CUDA_OK(cudaGetSymbolAddress((void **)&part, p2_noalloc_scratch),
+		"phase2_norm2_noalloc: scratch address");
 	int sms = 0;
 	if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
 			cudaSuccess ||

@@ -38,17 +38,38 @@ def everything():
             out.append(p2.qdrift(n, t, d, 16, 40, 0.05, 9))
             out += p2.batch("trott", [dict(nqb=n, terms=t, dets=d, steps=2,
                                            delta=0.1)] * 3)
+    out.append(norm())
     th = threading.Thread(target=lambda: register(8, p2.PREC_FP64))
     th.start()
     th.join()
     return out
 
-p2.world_ensure()
-want = everything()
+def norm():
+    # phase2_norm2_noalloc on a state of the process's own
+    st, res = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaMalloc(ctypes.byref(st), 16 << 10) == 0
+    assert rt.cudaMalloc(ctypes.byref(res), 16) == 0
+    host = np.arange(2 << 10, dtype=np.float64)
+    got = np.zeros(2)
+    assert rt.cudaMemcpy(st, host.ctypes.data_as(ctypes.c_void_p),
+                         ctypes.c_size_t(16 << 10), 1) == 0
+    fn = p2.lib().phase2_norm2_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64,
+                   ctypes.c_void_p, ctypes.c_void_p]
+    assert fn(st, p2.PREC_FP64, 1 << 10, res, None) == 0
+    assert rt.cudaMemcpy(got.ctypes.data_as(ctypes.c_void_p), res,
+                         ctypes.c_size_t(16), 2) == 0
+    assert rt.cudaFree(st) == 0 and rt.cudaFree(res) == 0
+    return got
+
 names = glob.glob(torch.__path__[0] + "/../nvidia/cuda_runtime/lib/"
                   "libcudart.so*") + ["libcudart.so.12"]
+rt = ctypes.CDLL(names[0])
+p2.world_ensure()
+want = everything()
+assert want[-1][0] == sum(k * k for k in range(2 << 10))
 for _ in range(2):
-    assert ctypes.CDLL(names[0]).cudaDeviceReset() == 0
+    assert rt.cudaDeviceReset() == 0
     for a, b in zip(want, everything()):
         assert np.array_equal(a, b)
 print("same")
