@@ -858,6 +858,7 @@ static void shell_free(struct p2_dev *d)
 		cudaEventDestroy(d->t1);
 	if (d->stream)
 		cudaStreamDestroy(d->stream);
+	cudaGetLastError(); /* of a shell made in part: not the next call's */
 	free(d);
 }
 

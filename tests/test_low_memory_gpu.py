@@ -67,6 +67,23 @@ except RuntimeError:
     print("done")
 """
 
+CREATION = """
+with Register(20, p2.PREC_FP64) as a:
+    held = leave(8)
+    made = []
+    try:
+        while True:
+            made.append(Register(14, p2.PREC_FP64))
+    except RuntimeError:
+        a.setamps([5], [2.0])
+        a.paulirot(np.array([5], dtype=np.uint64),
+                   np.array([0], dtype=np.uint64), np.array([0.0]))
+        assert a.norm2() == 4.0
+        print("done")
+    for r in made:
+        r.close()
+"""
+
 
 def _child(code):
     r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT,
@@ -84,3 +101,7 @@ def test_failed_register_keeps_nothing():
 
 def test_failure_stays_with_its_register():
     _child(FAILURE)
+
+
+def test_failed_creation_leaves_others_alone():
+    _child(CREATION)
