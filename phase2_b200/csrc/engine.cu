@@ -1739,13 +1739,20 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	const bool split = !brief && p2_split_ok(d, form);
 	const bool tile = !brief && p2_tile_ok(d, form, passes, npass, recs,
 		nrec);
-	const bool resident = split || tile ||
-		(!brief && !(d->nqb == 14 && npass == 2) &&
-			p2_resident_ok(d, form));
-	struct p2_graph *g = resident
+	const bool resident = !brief && !(d->nqb == 14 && npass == 2) &&
+		p2_resident_ok(d, form);
+	/* without room for its plan the flush runs on the pass kernels */
+	bool hit = false;
+	struct p2_graph *plan = tile || split || resident
+		? p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
+			  tile ? P2_PLAN_TILE
+				  : split ? P2_PLAN_SPLIT : P2_PLAN_RESIDENT,
+			  &hit)
+		: NULL;
+	struct p2_graph *g = plan
 		? NULL
 		: graph_for(d, passes, npass, recs, nrec);
-	if (!resident && !g) {
+	if (!plan && !g) {
 		if (recs_reserve(d, nrec) < 0)
 			return -1;
 		struct phase2_rot_rec *stage = p2_stage_reserve(d, nrec);
@@ -1756,20 +1763,17 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 			return -1;
 	}
 
-	if (d->timing && !resident)
+	if (d->timing)
 		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	long launches;
-	if (tile) {
-		size_t trips;
-		if (p2_tile_run(d, passes, npass, recs, nrec, plan_id,
-			    &trips) < 0)
+	if (plan && tile) {
+		if (p2_tile_run(d, plan) < 0)
 			return -1;
-		d->launches += trips;
-		launches = (long)trips;
-	} else if (resident) {
+		d->launches += plan->ntile;
+		launches = (long)plan->ntile;
+	} else if (plan) {
 		/* counted as one state round trip a pass, as planned */
-		if ((split ? p2_split_run : p2_resident_run)(d, passes, npass,
-			    recs, nrec, plan_id) < 0)
+		if ((split ? p2_split_run : p2_resident_run)(d, plan) < 0)
 			return -1;
 		d->launches += split ? npass : 1;
 		launches = (long)npass;
@@ -1784,7 +1788,8 @@ extern "C" int p2d_run(struct p2_dev *d, const struct phase2_pass *passes,
 	CUDA_OK(cudaGetLastError(), "pass launch");
 	d->passes += npass;
 	d->sweeps += (uint64_t)launches;
-	d->launches += resident ? 0 : (uint64_t)launches;
+	d->launches += plan ? 0 : (uint64_t)launches;
+	d->graph_replays += plan && hit;
 	d->rotations += nrec;
 	if (d->timing) {
 		CUDA_OK(cudaEventRecord(d->t1, d->stream), "timing stop");

@@ -225,16 +225,14 @@ int p2_stage_upload(struct p2_dev *d, void *dst, size_t bytes);
 void p2_graph_drop(struct p2_dev *d, struct p2_graph *g);
 
 /* resident.cu: whether a register's flush of this form runs as one launch
- * on the register held in shared memory, and that launch (between the
- * timing events; the caller counts it).  plan_id: nonzero and the same for
- * flushes with the same passes and records. */
+ * on the register held in shared memory, and that launch (the caller counts
+ * it). */
 bool p2_resident_ok(const struct p2_dev *d, int form);
-int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id);
+int p2_resident_run(struct p2_dev *d, const struct p2_graph *g);
 
 /* resident.cu: a register's plan slot for a flush, its sub-passes on the
- * device (see there). */
+ * device (see there); NULL where there is no room for them.  plan_id:
+ * nonzero and the same for flushes with the same passes and records. */
 enum p2_plan_kind { P2_PLAN_RESIDENT, P2_PLAN_SPLIT, P2_PLAN_TILE };
 struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	const struct phase2_pass *passes, size_t npass,
@@ -245,9 +243,7 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
  * whether a register's flush of this form runs there, and its launches, as
  * p2_resident_run. */
 bool p2_split_ok(const struct p2_dev *d, int form);
-int p2_split_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id);
+int p2_split_run(struct p2_dev *d, const struct p2_graph *g);
 
 /*
  * resident.cu: a round of samples run on chip, one cluster each: sample s's
@@ -319,14 +315,11 @@ cudaError_t p2_resident_progs(const struct p2_dev *d, uint32_t nqb, uint32_t g,
 	struct p2_bctl *ctl, unsigned long long *start);
 
 /* tile.cu: FP64 registers beyond the caches: whether a flush's rotations run
- * regrouped into tile runs, and their launches, as p2_resident_run; *trips:
- * state round trips. */
+ * regrouped into tile runs, and their launches, as p2_resident_run. */
 bool p2_tile_ok(const struct p2_dev *d, int form,
 	const struct phase2_pass *passes, size_t npass,
 	const struct phase2_rot_rec *recs, size_t nrec);
-int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id, size_t *trips);
+int p2_tile_run(struct p2_dev *d, const struct p2_graph *g);
 
 /* lift_bulk.cu: one FP32 pass of the FP64-arithmetic form on a kernel
  * whose next cosets are staged in shared memory, by bulk copies (variant

@@ -497,7 +497,7 @@ struct p2_graph *p2_sub_plan(struct p2_dev *d,
 	lru->used = d->graph_clock;
 	return lru;
 fail:
-	log_error("resident plan: out of memory");
+	log_warn("no room for a flush's sub-passes: pass kernels");
 	cudaGetLastError();
 	p2_graph_drop(d, lru);
 	return NULL;
@@ -606,18 +606,8 @@ static int res_launch_flush(struct p2_dev *d, const struct p2_graph *g)
 	return 0;
 }
 
-int p2_resident_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id)
+int p2_resident_run(struct p2_dev *d, const struct p2_graph *g)
 {
-	bool hit;
-	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
-		P2_PLAN_RESIDENT, &hit);
-	if (!g)
-		return -1;
-	d->graph_replays += hit;
-	if (d->timing)
-		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	return d->prec == PHASE2_PREC_FP64
 		? res_launch_flush<double2, false>(d, g)
 		: res_launch_flush<float2, true>(d, g);

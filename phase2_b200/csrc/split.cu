@@ -193,18 +193,8 @@ static int split_launch(struct p2_dev *d, const struct p2_graph *g)
 	return 0;
 }
 
-int p2_split_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id)
+int p2_split_run(struct p2_dev *d, const struct p2_graph *g)
 {
-	bool hit;
-	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
-		P2_PLAN_SPLIT, &hit);
-	if (!g)
-		return -1;
-	d->graph_replays += hit;
-	if (d->timing)
-		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	return d->prec == PHASE2_PREC_FP64 ? split_launch<double2, false>(d, g)
 					   : split_launch<float2, true>(d, g);
 }

@@ -250,16 +250,8 @@ bool p2_tile_ok(const struct p2_dev *d, int form,
 			short_gain(passes, npass, recs, nrec));
 }
 
-int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
-	size_t npass, const struct phase2_rot_rec *recs, size_t nrec,
-	uint64_t plan_id, size_t *trips)
+int p2_tile_run(struct p2_dev *d, const struct p2_graph *g)
 {
-	bool hit;
-	struct p2_graph *g = p2_sub_plan(d, passes, npass, recs, nrec, plan_id,
-		P2_PLAN_TILE, &hit);
-	if (!g)
-		return -1;
-	d->graph_replays += hit;
 	static uint64_t done;
 	unsigned per_sm;
 	if (!p2_done(&done, d->context, &per_sm)) {
@@ -278,15 +270,12 @@ int p2_tile_run(struct p2_dev *d, const struct phase2_pass *passes,
 	uint64_t grid = (uint64_t)d->sm_count * per_sm;
 	if (grid > ntile)
 		grid = ntile;
-	if (d->timing)
-		CUDA_OK(cudaEventRecord(d->t0, d->stream), "timing start");
 	const struct p2_tile_rec *r = (const struct p2_tile_rec *)g->d_recs;
-	const struct p2_tile_sub *s = (const struct p2_tile_sub *)(r + nrec);
+	const struct p2_tile_sub *s = (const struct p2_tile_sub *)(r + g->nrec);
 	for (uint32_t i = 0; i < g->ntile; i++)
 		CUDA_OK(p2_launch(k_tile, (unsigned)grid, P2_TILE_TPB,
 				P2_TILE_BYTES, d->stream, (double2 *)d->state,
 				ntile, g->tiles[i], s, r),
 			"tile launch");
-	*trips = g->ntile;
 	return 0;
 }

@@ -1,6 +1,7 @@
 """Little free device memory, in a child process that holds the rest: device
 sampling falls back on the kernel that needs less scratch, with the same
-bits, and a call that fails leaves other registers alone."""
+bits, a flush without room for its plan runs on the pass kernels, and a call
+that fails leaves other registers alone."""
 
 import subprocess
 import sys
@@ -85,6 +86,49 @@ with Register(20, p2.PREC_FP64) as a:
 """
 
 
+PLAN = """
+n, k = 21, 6000
+rng = np.random.Generator(np.random.PCG64(1))
+ops = (rng.integers(0, 1 << n, k).astype(np.uint64),
+       rng.integers(0, 1 << n, k).astype(np.uint64), rng.uniform(-1, 1, k))
+amp = np.zeros(1 << n, dtype=complex)
+amp[5] = 1.0
+with Register(n, p2.PREC_FP64) as r, Register(n, p2.PREC_FP64) as first:
+    # both kinds of kernel and the records' buffer, while there is room
+    first.set_state(amp)
+    first.paulirot(*ops)
+    want = first.get_state()
+    p2.lib().phase2_set_fp32_form(p2.FORM_LIFTED_F32)
+    with Register(n, p2.PREC_FP32) as f:
+        f.paulirot(*ops)
+        f.synchronize()
+    r.set_fusion(4, 0)
+    r.set_state(amp)
+    r.paulirot(*ops)
+    r.get_state()
+    r.set_fusion(5, 0)
+    r.set_state(amp)
+    # destroyed registers' streams and buffers for those made below
+    kept = [Register(10, p2.PREC_FP64) for _ in range(31)]
+    for x in kept:
+        x.close()
+    held = leave(8)
+    # then what the pool still has
+    rest, m = [], 22
+    while m >= 10 and len(rest) < 31:
+        try:
+            rest.append(Register(m, p2.PREC_FP64))
+        except RuntimeError:
+            m -= 1
+    r.paulirot(*ops)
+    assert np.array_equal(r.get_state(), want)
+    assert r.stats()["rotations"] == 2 * k
+    print("done")
+    for x in rest:
+        x.close()
+"""
+
+
 def _child(code):
     r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT,
                        timeout=600, capture_output=True, text=True)
@@ -93,6 +137,10 @@ def _child(code):
 
 def test_device_sampling_without_room_for_sub_passes():
     _child(SAMPLING)
+
+
+def test_flush_without_room_for_its_plan():
+    _child(PLAN)
 
 
 def test_failed_register_keeps_nothing():
